@@ -94,6 +94,8 @@ def _fits(c):
     if c["kind"] == "step" and M * (n // 2 + 1) * n * n * 16 > 62 * 2 ** 20:
         return False
     if c["prec"] == "fp64":
+        if n > 96:
+            return False
         return M * ((n + 1) * 16 + (n * 8 + 60 if c["lit"] == "real4" else 0)) < 215e3
     return M * (n + 1) * 8 < 220e3
 
