@@ -38,6 +38,14 @@ __host__ __device__ constexpr int xy_planes(int N, int tsize, int zd) {
     return (zd == 1 && z / 2 >= 1 && ((z / 2) * 2 * tsize) % 16 == 0) ? z / 2 : z;
 }
 
+// 16-bit exponents kept in shared memory by passes A and C of the FP64 form
+// (wlc_fixfft.cuh): between the sub-passes of the longer of the two line
+// batches, and one per line of the other
+__host__ __device__ constexpr int xy_exps(int N, int z, int zb) {
+    const int lx = zb * (N / 2), ly = z * (N / 2 + 1), r = N > 64 ? 16 : 8;
+    return (lx > ly ? lx : ly) * r + ly;
+}
+
 // StepArgs::order of a step of the operator-split scheme (WLC_SCHEME_SPLIT):
 // pass A multiplies q(s-1) by e^{-w ds/2} (cf / dsw hold that factor),
 // pass B applies the Crank-Nicolson operator, pass C multiplies by
@@ -115,6 +123,7 @@ template <typename T> struct SolveArgs {
 // the host launcher and the kernel.
 struct SolveSmem {
     size_t col, tw, csa, csaf, zoff, zofff, dr_ptr, dr_col, dr_axis, dr_valf, corr, masks;
+    size_t es;  // FP64 form: exponents between the sub-passes of the z-FFTs, in the space of corr where there is one
     size_t total;
 };
 
@@ -140,6 +149,7 @@ __host__ __device__ inline SolveSmem solve_smem(int N, int M, int L, int ndr, in
     s.dr_axis = take(correct ? (size_t)ndr : 0);
     s.dr_valf = take(correct ? 4 * (size_t)ndr : 0);
     s.corr = take(correct ? 8 * (size_t)M * N : 0);  // FP32 correction vectors [i][kz]
+    s.es = correct ? s.corr : take(tsize == 8 ? 2 * (size_t)M * (N > 64 ? 16 : 8) : 0);
     s.masks = take(4 * 2 * 32);                      // work split of the solve phase
     s.total = o;
     return s;

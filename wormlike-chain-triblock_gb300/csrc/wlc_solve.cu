@@ -14,6 +14,7 @@
 #include <cstdio>
 
 #include "wlc_attr.h"
+#include "wlc_fixfft.cuh"
 #include "wlc_kernels.cuh"
 #include "wlc_rot_gen.cuh"
 #include "wlc_step.h"
@@ -214,6 +215,8 @@ __global__ void __launch_bounds__(kSolveThreads, (sizeof(T) == 4) ? 2 : 1)
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C* col = reinterpret_cast<C*>(smem_raw + sm.col);
     C* tw = reinterpret_cast<C*>(smem_raw + sm.tw);
+    fxw* twx = reinterpret_cast<fxw*>(smem_raw + sm.tw);
+    int16_t* es = reinterpret_cast<int16_t*>(smem_raw + sm.es);
     T* csa = reinterpret_cast<T*>(smem_raw + sm.csa);
     float* csaf = reinterpret_cast<float*>(smem_raw + sm.csaf);
     T* s_zoff = reinterpret_cast<T*>(smem_raw + sm.zoff);
@@ -238,7 +241,11 @@ __global__ void __launch_bounds__(kSolveThreads, (sizeof(T) == 4) ? 2 : 1)
     const int kyi = colid / a.nkx, kxi = colid % a.nkx;
     const int ix = fold_n(kxi, N), iy = fold_n(kyi, N);
     const double kx = ix * a.kf[0], ky = iy * a.kf[1];
-    for (int e = threadIdx.x; e < N; e += blockDim.x) tw[e] = a.twg[e];
+    if constexpr (sizeof(T) == 8) {
+        for (int e = threadIdx.x; e < N; e += blockDim.x) twx[e] = make_fxw(a.twg[e]);
+    } else {
+        for (int e = threadIdx.x; e < N; e += blockDim.x) tw[e] = a.twg[e];
+    }
     if (threadIdx.x == 0) {
         const double rho = sqrt(kx * kx + ky * ky);
         const double ca = rho > 0 ? kx / rho : 1.0, sa = rho > 0 ? ky / rho : 0.0;
@@ -255,7 +262,10 @@ __global__ void __launch_bounds__(kSolveThreads, (sizeof(T) == 4) ? 2 : 1)
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
-    fft_nat2perm<N, -1>(col, M, 1, NP, tw);
+    if constexpr (sizeof(T) == 8)
+        fx_nat2perm<N, -1, true>(col, M, 1, NP, twx, es, es, FromDoubles{});
+    else
+        fft_nat2perm<N, -1>(col, M, 1, NP, tw);
 
     // Work split: thread t owns kz position p = t % N and part t / N of its
     // solve (a greedy balance of the degree blocks and of the m systems
@@ -361,7 +371,10 @@ __global__ void __launch_bounds__(kSolveThreads, (sizeof(T) == 4) ? 2 : 1)
         }
     }
     __syncthreads();
-    fft_perm2nat<N, +1>(col, M, 1, NP, tw);
+    if constexpr (sizeof(T) == 8)
+        fx_perm2nat<N, +1, true>(col, M, 1, NP, twx, es, es, FromDoubles{});
+    else
+        fft_perm2nat<N, +1>(col, M, 1, NP, tw);
     if (a.split) {
         // Crank-Nicolson operator (I + ds/2 A)^-1 (I - ds/2 A) = 2 (I + ds/2 A)^-1 - I
         // applied through the z transforms: IFFT_z(2x - b) = 2 IFFT_z(x) - N b,

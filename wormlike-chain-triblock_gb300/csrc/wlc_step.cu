@@ -4,6 +4,7 @@
 #include <cstdio>
 
 #include "wlc_attr.h"
+#include "wlc_fixfft.cuh"
 #include "wlc_kernels.cuh"
 #include "wlc_step.h"
 
@@ -119,6 +120,25 @@ __device__ __forceinline__ void fwd_x_planes(typename cvec<T>::t* zb, typename c
     __syncthreads();
 }
 
+// the same in the FP64 form: fixed-point half spectra (twice their value)
+// with one exponent per row pair in el
+template <int N, int Z, int ZB>
+__device__ __forceinline__ void fwd_x_planes_fx(double2* zb, fxc* out, int zz0, const fxw* tw, int16_t* es, int16_t* el) {
+    constexpr int NKX = N / 2 + 1;
+    constexpr int XR = xrow(N);
+    fx_nat2perm<N, -1, false>(zb, ZB * (N / 2), 1, XR, tw, es, el + zz0 * (N / 2), FromDoubles{});
+    for (int t = threadIdx.x; t < ZB * (N / 2) * NKX; t += blockDim.x) {
+        const int q = t / ((N / 2) * NKX), e = t % ((N / 2) * NKX);
+        const int p = e / NKX, k = e % NKX;
+        const fxc* zq = reinterpret_cast<const fxc*>(zb) + (size_t)q * xplane(N);
+        const fxc zk = zq[p * XR + perm_pos<N>(k)];
+        const fxc zm = zq[p * XR + perm_pos<N>((N - k) % N)];
+        out[((2 * p) * NKX + k) * Z + zz0 + q] = fxc{zk.x + zm.x, zk.y - zm.y};
+        out[((2 * p + 1) * NKX + k) * Z + zz0 + q] = fxc{zk.y + zm.y, zm.x - zk.x};
+    }
+    __syncthreads();
+}
+
 // y-FFTs of every (kx, plane) line of out: line kx*Z + zz starts at out + kx*Z + zz,
 // element ky at stride NKX*Z
 template <typename T, int N, int Z, int DIR>
@@ -162,6 +182,7 @@ __global__ void __launch_bounds__(512) rhs_fft_xy(StepArgs<T> a0, const StepArgs
     const StepArgs<T> a = pick_args<B>(a0, batch);
     using C = typename cvec<T>::t;
     constexpr int Z = XyShape<T, N, V>::Z, ZB = XyShape<T, N, V>::ZB;
+    constexpr int NKX = N / 2 + 1;
     constexpr int NR = N * N * N;
     constexpr int PB = (N / 2) * N;  // packed row pairs per plane
     constexpr int XR = xrow(N), PBS = xplane(N);
@@ -171,7 +192,14 @@ __global__ void __launch_bounds__(512) rhs_fft_xy(StepArgs<T> a0, const StepArgs
     C* out = zb + (size_t)ZB * PBS;  // N x NKX x Z half spectra
     const int i = blockIdx.y;
     const int z0 = blockIdx.x * Z;
-    for (int e = threadIdx.x; e < N; e += blockDim.x) tw[e] = a.twg[e];
+    fxw* twx = reinterpret_cast<fxw*>(smem_raw);
+    int16_t* el = reinterpret_cast<int16_t*>(out + (size_t)Z * N * NKX);  // FP64 form: exponents per line, then scratch
+    int16_t* es = el + Z * NKX;
+    if constexpr (sizeof(T) == 8) {
+        for (int e = threadIdx.x; e < N; e += blockDim.x) twx[e] = make_fxw(a.twg[e]);
+    } else {
+        for (int e = threadIdx.x; e < N; e += blockDim.x) tw[e] = a.twg[e];
+    }
     for (int zz0 = 0; zz0 < Z; zz0 += ZB) {
         if constexpr (sizeof(T) == 4) {
             // four consecutive x per thread: 16-byte loads of the history, ds*w
@@ -205,9 +233,17 @@ __global__ void __launch_bounds__(512) rhs_fft_xy(StepArgs<T> a0, const StepArgs
             }
         }
         __syncthreads();
-        fwd_x_planes<T, N, Z, ZB>(zb, out, zz0, tw);
+        if constexpr (sizeof(T) == 8)
+            fwd_x_planes_fx<N, Z, ZB>(zb, reinterpret_cast<fxc*>(out), zz0, twx, es, el);
+        else
+            fwd_x_planes<T, N, Z, ZB>(zb, out, zz0, tw);
     }
-    y_planes<T, N, Z, -1>(out, tw);
+    if constexpr (sizeof(T) == 8)  // the half spectra hold twice their value: exponent - 1
+        fx_nat2perm<N, -1, true>(out, NKX * Z, NKX * Z, 1, twx, es, es, from_fixed([=](int line, int y) {
+                                     return el[(line % Z) * (N / 2) + (y >> 1)] - 1;
+                                 }));
+    else
+        y_planes<T, N, Z, -1>(out, tw);
     store_phat<T, N, Z>(a, out, i, z0);
 }
 
@@ -290,6 +326,11 @@ __global__ void __launch_bounds__(512) rhs_fft_xy_staged(StepArgs<float> a0, con
 }
 
 // ---------------------------------------------------------------- pass C
+__host__ __device__ constexpr int ilog2(int n) { return n > 1 ? 1 + ilog2(n / 2) : 0; }
+// what the y-FFTs of pass C leave: fixed-point numbers in the FP64 form
+template <typename T> struct KspaceElem { using t = float2; };
+template <> struct KspaceElem<double> { using t = fxc; };
+
 template <typename T, int N, bool B = false, int V = 0>
 __global__ void __launch_bounds__(512) ifft_xy(StepArgs<T> a0, const StepArgs<T>* __restrict__ batch) {
     const StepArgs<T> a = pick_args<B>(a0, batch);
@@ -306,7 +347,17 @@ __global__ void __launch_bounds__(512) ifft_xy(StepArgs<T> a0, const StepArgs<T>
     C* out = zb + (size_t)ZB * PBS;
     const int i = blockIdx.y;
     const int z0 = blockIdx.x * Z;
-    for (int e = threadIdx.x; e < N; e += blockDim.x) tw[e] = a.twg[e];
+    fxw* twx = reinterpret_cast<fxw*>(smem_raw);
+    int16_t* el = reinterpret_cast<int16_t*>(out + (size_t)Z * N * NKX);  // FP64 form: exponents per line, then scratch
+    int16_t* es = el + Z * NKX;
+    if constexpr (sizeof(T) == 8) {
+        for (int e = threadIdx.x; e < N; e += blockDim.x) twx[e] = make_fxw(a.twg[e]);
+    } else {
+        for (int e = threadIdx.x; e < N; e += blockDim.x) tw[e] = a.twg[e];
+    }
+    // 1/N^3 is a shift of the exponents where N is a power of two
+    constexpr bool kPow2 = sizeof(T) == 8 && (N & (N - 1)) == 0;
+    constexpr int kShift = kPow2 ? 3 * ilog2(N) : 0;
     // all loads issued up front: one Z-run (Z * sizeof(C) bytes) per (ky, kx)
     constexpr int CH = (Z * (int)sizeof(C)) / 16;  // 16-byte chunks per run
     static_assert((Z * sizeof(C)) % 16 == 0, "phat runs must be whole 16-byte chunks");
@@ -319,7 +370,11 @@ __global__ void __launch_bounds__(512) ifft_xy(StepArgs<T> a0, const StepArgs<T>
     cp_async_commit();
     cp_async_wait<0>();
     __syncthreads();
-    y_planes<T, N, Z, +1>(out, tw);  // along y for every plane; row y now at perm_pos(y)
+    // along y for every plane; row y now at perm_pos(y)
+    if constexpr (sizeof(T) == 8)
+        fx_nat2perm<N, +1, false>(out, NKX * Z, NKX * Z, 1, twx, es, el, FromDoubles{});
+    else
+        y_planes<T, N, Z, +1>(out, tw);
     for (int zz0 = 0; zz0 < Z; zz0 += ZB) {
         // Hermitian extension of rows (2p, 2p+1) packed as one complex row;
         // the imaginary parts at kx = 0 and N/2 are discarded (c2r)
@@ -329,15 +384,16 @@ __global__ void __launch_bounds__(512) ifft_xy(StepArgs<T> a0, const StepArgs<T>
             const int q = t % ZB, e = t / ZB;
             const int zz = zz0 + q;
             const int p = e / N, k = e % N;
-            const C* ra = out + (size_t)perm_pos<N>(2 * p) * NKX * Z + zz;
-            const C* rb = out + (size_t)perm_pos<N>(2 * p + 1) * NKX * Z + zz;
-            C xa, xb;
+            using K = typename KspaceElem<T>::t;
+            const K* ra = reinterpret_cast<const K*>(out) + (size_t)perm_pos<N>(2 * p) * NKX * Z + zz;
+            const K* rb = reinterpret_cast<const K*>(out) + (size_t)perm_pos<N>(2 * p + 1) * NKX * Z + zz;
+            K xa, xb;
             if (k <= N / 2) {
                 xa = ra[k * Z];
                 xb = rb[k * Z];
                 if (k == 0 || k == N / 2) {
-                    xa.y = (T)0;
-                    xb.y = (T)0;
+                    xa.y = decltype(xa.y)(0.0);
+                    xb.y = decltype(xb.y)(0.0);
                 }
             } else {
                 xa = ra[(N - k) * Z];
@@ -345,23 +401,30 @@ __global__ void __launch_bounds__(512) ifft_xy(StepArgs<T> a0, const StepArgs<T>
                 xa.y = -xa.y;
                 xb.y = -xb.y;
             }
-            zb[(size_t)q * PBS + p * XR + k] = cmk<C>(xa.x - xb.y, xa.y + xb.x);
+            reinterpret_cast<K*>(zb)[(size_t)q * PBS + p * XR + k] = cmk<K>(xa.x - xb.y, xa.y + xb.x);
         }
         __syncthreads();
-        fft_nat2perm<N, +1>(zb, ZB * (N / 2), 1, XR, tw);  // along x; x at perm_pos(x)
+        // along x; x at perm_pos(x)
+        if constexpr (sizeof(T) == 8)
+            fx_nat2perm<N, +1, true>(zb, ZB * (N / 2), 1, XR, twx, es, es, from_fixed([=](int line, int k) {
+                                         return el[(k <= N / 2 ? k : N - k) * Z + zz0 + line / (N / 2)] - kShift;
+                                     }));
+        else
+            fft_nat2perm<N, +1>(zb, ZB * (N / 2), 1, XR, tw);
         // packed row pair p holds rows 2p (real part) and 2p+1 (imaginary part)
         for (int t = threadIdx.x; t < ZB * PB; t += blockDim.x) {
             const int q = t / PB, e = t % PB;
             const int p = e / N, x = e % N;
-            const C v = zb[(size_t)q * PBS + p * XR + perm_pos<N>(x)];
+            C v = zb[(size_t)q * PBS + p * XR + perm_pos<N>(x)];
+            if constexpr (!kPow2) v = cscale(v, a.minv);
             const size_t r = (size_t)(z0 + zz0 + q) * N * N + (size_t)(2 * p) * N + x;
             T* dst = a.qout + (size_t)i * NR + r;
             if (a.post) {  // split scheme: the second field half step
-                dst[0] = (v.x * a.minv) * a.post[r];
-                dst[N] = (v.y * a.minv) * a.post[r + N];
+                dst[0] = v.x * a.post[r];
+                dst[N] = v.y * a.post[r + N];
             } else {
-                dst[0] = v.x * a.minv;
-                dst[N] = v.y * a.minv;
+                dst[0] = v.x;
+                dst[N] = v.y;
             }
         }
         __syncthreads();
@@ -381,7 +444,8 @@ __global__ void __launch_bounds__(256) rhs_only(StepArgs<T> a, T* out) {
 template <typename T> size_t smem_xy(int N, int variant) {
     using C = typename cvec<T>::t;
     const int z = xy_planes(N, sizeof(T), variant & 1), zb = (variant & 2) ? z : 1;
-    return sizeof(C) * ((size_t)N + (size_t)zb * xplane(N) + (size_t)z * N * (N / 2 + 1));
+    return sizeof(C) * ((size_t)N + (size_t)zb * xplane(N) + (size_t)z * N * (N / 2 + 1)) +
+           (sizeof(T) == 8 ? 2 * (size_t)xy_exps(N, z, zb) : 0);
 }
 
 // shared-memory limits of the pass A / pass C kernels of (T, N, B), once per
