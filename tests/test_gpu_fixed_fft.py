@@ -62,3 +62,22 @@ def test_non_finite_input_stays_non_finite(n, bad):
     q = g.mde_one_step(3, pr)
     assert np.isnan(q[:, 0]).all()
     g.close()
+
+
+def test_rotations_without_room_for_their_table():
+    """N = 96, L = 11 with real-8 literals is the one size whose column leaves
+    no shared memory for the table of cos, sin(m beta) (the rotations then run
+    on doubles): one step against the FP32 form, whose rounding (2^-24 an
+    operation, some hundred operations in sequence) bounds the difference."""
+    n, L = 96, 11
+    rng = np.random.default_rng(5)
+    M, nr = (L + 1) ** 2, n ** 3
+    pr = rng.standard_normal((nr, 1), dtype=np.float32) * rng.uniform(0.1, 1.0, size=(1, M)).astype(np.float32)
+    pr = pr.astype(np.float64)
+    q = []
+    for precision in (wlc.WLC_FP64, wlc.WLC_FP32):
+        g = wlc.Instance(n, L, 10, (4, 2, 4), 1.2 / n, 1.3, (0.5, 0.6, 0.7), (15.0,) * 3, literals=wlc.WLC_LIT_REAL8,
+                         precision=precision, store_qstar=0, q_checkpoint=3)
+        q.append(g.mde_one_step(7, pr))
+        g.close()
+    assert np.abs(q[0] - q[1]).max() < 200 * 2.0 ** -24 * np.abs(q[0]).max()

@@ -6,7 +6,8 @@ the rotation by +pi/2 about x with a fixed (2l+1)x(2l+1) orthogonal matrix
 X_l (about a quarter of its entries are nonzero); X_l^T undoes it.  The
 factorised solve applies X_l and X_l^T four times per wavevector, so the
 codelets unroll them into straight-line FMAs on register arrays (no table
-loads).  The entries are computed here by exact Gauss-Legendre x uniform
+loads); the FP64 form's solve takes the same matrices block by block from tables of
+fixed-point factors.  The entries are computed here by exact Gauss-Legendre x uniform
 quadrature of products of real harmonics, with the harmonic convention the
 reference uses (checked against its triple products in the tests).
 
@@ -94,17 +95,84 @@ def rotation_x90(l):
             for i in range(n):
                 for j in range(n):
                     X[i][j] += wq * Y[i] * Y2[j]
-    Xd = np.array([[float(X[i][j]) if abs(X[i][j]) > mp.mpf(10) ** (-25) else 0.0 for j in range(n)]
-                   for i in range(n)])
-    return Xd
+    return [[v if abs(v) > mp.mpf(10) ** (-25) else mp.mpf(0) for v in row] for row in X]
+
+
+def to_double(X):
+    return np.array([[float(v) for v in row] for row in X])
+
+
+def classes(X, l):
+    """The four dense blocks of X_l: (outputs, inputs), both with stride 2 in j = m + l."""
+    n = 2 * l + 1
+    out = []
+    seen = set()
+    for j in range(n):
+        if j in seen:
+            continue
+        rows, cols = [j], []
+        while True:  # the connected component of row j (single entries of a block may vanish)
+            c2 = [m for m in range(n) if any(X[r][m] != 0 for r in rows)]
+            r2 = [r for r in range(n) if any(X[r][c] != 0 for c in c2)]
+            if (r2, c2) == (rows, cols):
+                break
+            rows, cols = r2, c2
+        assert len(rows) == len(cols)
+        assert all(b - a == 2 for q in (rows, cols) for a, b in zip(q, q[1:]))
+        seen.update(rows)
+        out.append((rows, cols))
+    return out
+
+
+def halves(v):
+    """v * 2^62 as h 2^32 + l with both halves signed."""
+    q = int(mp.nint(v * mp.mpf(2) ** 62))
+    l = ((q + 2 ** 31) % 2 ** 32) - 2 ** 31
+    return (q - l) >> 32, l
+
+
+def emit_blocks(Xs):
+    """The dense blocks as tables of fixed-point factors, for X and for its transpose."""
+    tabs, desc, shift = ([], []), [], []
+    for l, X in enumerate(Xs):
+        d, sh = [], [[0, 0], [0, 0]]
+        for rows, cols in classes(X, l):
+            d.append((len(rows), cols[0], len(tabs[0])))
+            for r in rows:
+                tabs[0].extend(halves(X[r][c]) for c in cols)
+            for c in cols:
+                tabs[1].extend(halves(X[r][c]) for r in rows)
+            for r, c in zip(rows, cols):  # output r is kept in the slot of input c
+                m = r - l
+                sh[abs(m) % 2][0 if m >= 0 else 1] = c - r
+        while len(d) < 4:
+            d.append((0, 0, 0))
+        desc.append(d)
+        shift.append(sh)
+    n = len(tabs[0])
+    out = ["// X_l falls into four dense blocks on every second element.  kXdesc[l][b]:",
+           "// size, first input element and place in kXtab of block b; the outputs are",
+           "// written over the inputs.  kXshift[l][m odd][sin part]: where output (l, m)",
+           "// or (l, -m) then lies, less its own place.  kXtab: factors of 62 fraction bits",
+           "// as signed halves {h, l}, row by row, X (first half) and its transpose.",
+           "constexpr int kXentries = %d;" % n,
+           "__constant__ short kXdesc[%d][4][3] = {" % len(Xs)]
+    out += ["    {%s}," % ", ".join("{%d, %d, %d}" % b for b in d) for d in desc]
+    out += ["};", "__constant__ short kXshift[%d][2][2] = {" % len(Xs)]
+    out += ["    {{%d, %d}, {%d, %d}}," % (a[0], a[1], b[0], b[1]) for a, b in shift]
+    out += ["};", "__constant__ int2 kXtab[%d] = {" % (2 * n)]
+    flat = tabs[0] + tabs[1]
+    for i in range(0, len(flat), 4):
+        out.append("    " + " ".join("{%d, %d}," % t for t in flat[i:i + 4]))
+    out += ["};", ""]
+    return out
 
 
 def emit_apply(name, X, l):
     n = 2 * l + 1
-    lines = ["    template <typename T, typename C> __device__ __forceinline__ static void %s(const C* v, C* u) {" % name]
+    lines = ["    template <class A> __device__ __forceinline__ static void %s(const typename A::in* v, typename A::out* u) {" % name]
     # X maps each x-parity class onto itself: emit one class after the
     # other so the inputs of the first class die early (register pressure)
-    order = sorted(range(n), key=lambda j: (min([m for m in range(n) if X[j, m] != 0.0] or [0]) % 2, j))
     cls = {}
     for j in range(n):
         nz = [m for m in range(n) if X[j, m] != 0.0]
@@ -112,16 +180,11 @@ def emit_apply(name, X, l):
     order = sorted(range(n), key=lambda j: (cls[j], j))
     for j in order:
         terms = [(X[j, m], m) for m in range(n) if X[j, m] != 0.0]
-        if not terms:
-            lines.append("        u[%d] = cmk<C>((T)0, (T)0);" % j)
-            continue
         c, m = terms[0]
-        ex = "(T)%.17g * v[%d].x" % (c, m)
-        ey = "(T)%.17g * v[%d].y" % (c, m)
+        ex = "A::mul(%.17g, v[%d])" % (c, m)
         for c, m in terms[1:]:
-            ex = "fma((T)%.17g, v[%d].x, %s)" % (c, m, ex)
-            ey = "fma((T)%.17g, v[%d].y, %s)" % (c, m, ey)
-        lines.append("        u[%d] = cmk<C>(%s, %s);" % (j, ex, ey))
+            ex = "A::mad(%s, %.17g, v[%d])" % (ex, c, m)
+        lines.append("        u[%d] = A::done(%s);" % (j, ex))
     lines.append("    }")
     return lines
 
@@ -133,7 +196,8 @@ def main():
         "// wlc_rot_gen.cuh -- GENERATED by gen_rotation.py; do not edit.",
         "// Rotation by +pi/2 about x of the real-harmonic block l (XRot<l>::p,",
         "// u = X_l v) and its transpose (XRot<l>::m, u = X_l^T v), l = 0..%d," % lmax,
-        "// as straight-line FMAs on register arrays v[2l+1], u[2l+1] (index m+l).",
+        "// as straight-line sums on register arrays v[2l+1], u[2l+1] (index m+l); A",
+        "// gives the arithmetic (product, product added to a sum, the sum's result).",
         "#pragma once",
         '#include "wlc_fft.cuh"',
         "",
@@ -143,8 +207,9 @@ def main():
         "",
     ]
     total = 0
+    exact = [rotation_x90(l) for l in range(lmax + 1)]
     for l in range(lmax + 1):
-        X = rotation_x90(l)
+        X = to_double(exact[l])
         assert np.abs(X @ X.T - np.eye(2 * l + 1)).max() < 1e-13
         total += int((X != 0).sum())
         out.append("template <> struct XRot<%d> {" % l)
@@ -153,6 +218,10 @@ def main():
         out.append("};")
         out.append("")
     out.append("constexpr int kRotLmax = %d;" % lmax)
+    out.append("")
+    out.append("#ifdef WLC_ROT_TABLES")
+    out += emit_blocks(exact)
+    out.append("#endif")
     out.append("")
     out.append("}  // namespace wlc")
     path = os.path.join(here, "wlc_rot_gen.cuh")

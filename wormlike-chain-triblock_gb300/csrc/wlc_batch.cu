@@ -185,6 +185,7 @@ static int batch_issue_group(wlc_batch* b, wlc_batch::Group& g, cudaStream_t st)
         bl.count = cnt;
         bl.M = b->M;
         bl.nkx = g.N / 2 + 1;
+        bl.lmax = b->inst[g.idx[0]]->L;
         bl.solve_smem = g.smem;
         bl.a_variant = g.a_variant;
         bl.solve_threads = g.solve_threads;
@@ -406,6 +407,7 @@ extern "C" int wlc_batch_autotune(wlc_batch* b, int32_t* config) {
                 bl.count = cnt;
                 bl.M = b->M;
                 bl.nkx = g.N / 2 + 1;
+                bl.lmax = b->inst[g.idx[0]]->L;
                 bl.solve_smem = g.smem;
                 bl.a_variant = av;
                 bl.solve_threads = th;

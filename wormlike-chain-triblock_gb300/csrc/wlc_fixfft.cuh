@@ -58,6 +58,7 @@ struct fxh {
 __device__ __forceinline__ fxh halves(long long v) {
     return {(int)(v >> 32) + (int)((unsigned)v >> 31), (int)(unsigned)v};
 }
+__device__ __forceinline__ long long join_halves(fxh a) { return ((long long)a.h << 32) + a.l; }
 // hi*2^64 + mid*2^32 -> units of 2^62 (the product with a constant of 62
 // fraction bits); the middle sums start from kHalf, so that the shift rounds
 constexpr long long kHalf = 1LL << 29;
@@ -113,18 +114,35 @@ __device__ __forceinline__ long long sar_s64(long long v, int s) {  // sign for 
 }
 // v / 2^s to the nearest, s >= 1 (halves up; 0 or so for s > 64)
 __device__ __forceinline__ long long round_shift(long long v, int s) { return (sar_s64(v, s - 1) + 1) >> 1; }
-// d as a fixed-point number under exponent E >= d's own
-__device__ __forceinline__ fx d2fx(double d, int E) {
+// d as a fixed-point number under exponent E >= d's own (E's leading bit at TOP)
+template <int TOP = kTop> __device__ __forceinline__ fx d2fx(double d, int E) {
     const int hi = __double2hiint(d), lo = __double2loint(d);
     const int s = E - ((hi >> 20) & 0x7ff);
     const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;
-    const unsigned long long m = (((unsigned long long)mh << 32) | (unsigned)lo) << (kTop - 51);
+    const unsigned long long m = (((unsigned long long)mh << 32) | (unsigned)lo) << (TOP - 51);
     const long long v = (long long)((shr_u64(m, s) + 1) >> 1);
     const long long sg = (long long)(hi >> 31);
     return mkfx((v ^ sg) - sg);
 }
 static __device__ __noinline__ double fx2d_rare(long long v, int E) {
     return E >= kExpBad / 2 ? __longlong_as_double(0x7ff8000000000000LL) : ldexp((double)v, E - 1023 - kTop);
+}
+// d as a float, round to nearest even, on the integer ALUs (the conversion
+// instruction runs on the FP64 pipe); below 2^-126 zero
+__device__ __forceinline__ float d2f(double d) {
+    const long long b = __double_as_longlong(d);
+    const long long r = b + 0x0fffffff + ((b >> 29) & 1);
+    const int e = (int)((r >> 52) & 0x7ff) - (1023 - 127);
+    const unsigned m = (unsigned)(r >> 29) & 0x7fffffu, sg = (unsigned)(b >> 32) & 0x80000000u;
+    return __uint_as_float(e <= 0 ? sg : e >= 255 ? sg | 0x7f800000u | ((b << 1) > (0x7ffLL << 53) ? 1u : 0u)
+                                                  : sg | ((unsigned)e << 23) | m);
+}
+// v under exponent E as a double by the conversion instruction: fewer
+// instructions than fx2d, on the FP64 pipe (for loops whose other work is on
+// the integer ALUs)
+__device__ __forceinline__ double fx2d_cvt(long long v, int E) {
+    const double d = __ll2double_rn(v);
+    return v == 0 ? 0.0 : __hiloint2double(__double2hiint(d) + ((E - 1023 - kTop) << 20), __double2loint(d));
 }
 // value of v under exponent E as a double (round to nearest, halves to even)
 __device__ __forceinline__ double fx2d(fx q, int E) {
@@ -178,11 +196,25 @@ template <int N> __host__ __device__ constexpr int fx_exps(int nlines) {
     return Plan<N>::N2 == 1 ? 0 : nlines * (Plan<N>::N1 > Plan<N>::N2 ? Plan<N>::N1 : Plan<N>::N2);
 }
 
-// Input of a line FFT: doubles, or fixed-point numbers with an exponent per
+// a float as a fixed-point number under exponent E >= fexp(f); subnormals count
+// as zero
+__device__ __forceinline__ int fexp(float f) { return ((__float_as_int(f) >> 23) & 0xff) + (1023 - 127); }
+__device__ __forceinline__ fx f2fx(float f, int E) {
+    const int u = __float_as_int(f), e = (u >> 23) & 0xff;
+    const long long m = (long long)((u & 0x7fffff) | 0x800000) << (kTop - 22);
+    const long long v = e == 0 ? 0 : round_shift(m, E - fexp(f) + 1);
+    return mkfx(u < 0 ? -v : v);
+}
+
+// Input of a line FFT: doubles, doubles less a correction in floats, or fixed-point numbers with an exponent per
 // (line, element).
 struct FromDoubles {
-    static constexpr bool dbl = true;
-    __device__ int operator()(int, int) const { return 0; }
+    static constexpr bool dbl = true, less = false;
+};
+struct FromDoublesLess {  // correction of (line, element) at c[line * stride + element]
+    static constexpr bool dbl = true, less = true;
+    const float2* c;
+    int stride;
 };
 template <typename F> struct FromFixed {
     static constexpr bool dbl = false;
@@ -198,11 +230,24 @@ __device__ __forceinline__ int fx_load(const double2* ln, int estride, int b, in
         double2 d[R];
 #pragma unroll
         for (int n = 0; n < R; ++n) d[n] = ln[(base + n * step) * estride];
-        const int E = shared_exp<R>(d);
+        int E = shared_exp<R>(d);
+        float2 c[In::less ? R : 1];
+        if constexpr (In::less) {
+#pragma unroll
+            for (int n = 0; n < R; ++n) {
+                c[n] = in.c[b * in.stride + base + n * step];
+                E = max(E, max(fexp(c[n].x), fexp(c[n].y)));
+            }
+            E = E < kExpBad ? E + 1 : E;  // room for the difference
+        }
 #pragma unroll
         for (int n = 0; n < R; ++n) {
             v[n].x = d2fx(d[n].x, E);
             v[n].y = d2fx(d[n].y, E);
+            if constexpr (In::less) {
+                v[n].x = v[n].x - f2fx(c[n].x, E);
+                v[n].y = v[n].y - f2fx(c[n].y, E);
+            }
         }
         return E;
     } else {

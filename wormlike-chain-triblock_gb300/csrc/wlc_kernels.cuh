@@ -122,8 +122,12 @@ template <typename T> struct SolveArgs {
 // Shared-memory carve-up of the solve kernel (bytes, 16-aligned), shared by
 // the host launcher and the kernel.
 struct SolveSmem {
-    size_t col, tw, csa, csaf, zoff, zofff, dr_ptr, dr_col, dr_axis, dr_valf, corr, masks;
-    size_t es;  // FP64 form: exponents between the sub-passes of the z-FFTs, in the space of corr where there is one
+    size_t col, tw, csa, csaf, zoff, zofff, dr_ptr, dr_col, dr_valf, corr;
+    // FP64 form: exponents between the sub-passes of the z-FFTs; cos, sin(m
+    // beta) [L+1][N] as fixed-point factors, in the space of corr where there
+    // is one (0: no room, the rotations then run on doubles -- only at N = 96,
+    // L = 11 with real-8 literals)
+    size_t es, beta;
     size_t total;
 };
 
@@ -146,16 +150,26 @@ __host__ __device__ inline SolveSmem solve_smem(int N, int M, int L, int ndr, in
     s.zofff = take(correct ? 4 * (size_t)M : 0);
     s.dr_ptr = take(correct ? 4 * (size_t)(M + 1) : 0);
     s.dr_col = take(correct ? 2 * (size_t)ndr : 0);
-    s.dr_axis = take(correct ? (size_t)ndr : 0);
     s.dr_valf = take(correct ? 4 * (size_t)ndr : 0);
     s.corr = take(correct ? 8 * (size_t)M * N : 0);  // FP32 correction vectors [i][kz]
-    s.es = correct ? s.corr : take(tsize == 8 ? 2 * (size_t)M * (N > 64 ? 16 : 8) : 0);
-    s.masks = take(4 * 2 * 32);                      // work split of the solve phase
+    s.es = take(tsize == 8 ? 2 * (size_t)M * (N > 64 ? 16 : 8) : 0);
+    const size_t nbeta = tsize == 8 ? 16 * (size_t)(L + 1) * N : 0;
+    s.beta = 0;
+    if (correct && 8 * (size_t)M * N >= nbeta)
+        s.beta = s.corr;
+    else if (tsize == 8 && o + nbeta <= 227 * 1024)
+        s.beta = take(nbeta);
     s.total = o;
     return s;
 }
 
-constexpr int kSolveThreads = 256;  // threads per CTA of the solve kernel (kz x parts in the solve phase)
+constexpr int kSolveThreads = 256;  // kz x parts of the solve phase at most (twice that many threads a CTA)
+constexpr int kSolveParts = kSolveThreads / 8;
+// degree blocks l of each part of the rotations, systems m of each part of
+// the tridiagonal sweeps (bit masks)
+struct SolveSplit {
+    uint16_t l[kSolveParts], m[2 * kSolveParts];
+};
 
 // Kernel arguments of one launch: the by-value parameter, or (batched
 // launches over several instances) entry blockIdx.z of a device array.

@@ -27,7 +27,7 @@ template <typename T> struct StepLaunch {
 template <typename T> struct BatchLaunch {
     const StepArgs<T>* dstep = nullptr;
     const SolveArgs<T>* dsolve = nullptr;
-    int count = 0, M = 0, nkx = 0;
+    int count = 0, M = 0, nkx = 0, lmax = 0;
     size_t solve_smem = 0;
     int a_variant = 0, solve_threads = 0, xy_threads = 0, xy_z = 0;
 };
