@@ -237,14 +237,15 @@ int wlc_last_timing(const wlc_ctx* ctx, double* ms4);
 
 /* No counterpart in the reference.  Launch autotuning: time the candidate
  * launch configurations of one contour step on this context's own data
- * (pass A variant, threads per solve CTA; all give identical results) and
+ * (passes A and C, threads per solve CTA; all give identical results) and
  * keep the fastest.  Runs a forward sweep first if none is current.
  * config (may be NULL) receives {a_variant, solve_threads, xy_threads,
- * xy_variant} (pass A variant 1 generic / 2 staged; threads per solve CTA;
- * threads per CTA of the generic pass A and pass C, 256 or 512; their
- * variant: bit 0 half the default number of z planes per CTA, bit 1 the
+ * xy_variant} (a_variant: always 1; kz positions x parts of a solve CTA,
+ * which has twice as many threads; threads per CTA of passes A and C, 256 or
+ * 512; their variant: bit 0 half the default number of z planes per CTA, bit 1 the
  * x-FFTs of all planes in one batched call).
- * wlc_set_launch_config sets them by hand (0, 0, 0, 0 = defaults). */
+ * wlc_set_launch_config sets them by hand (0, 0, 0, 0 = by size; a_variant
+ * 0..2 are accepted and the same). */
 int wlc_autotune(wlc_ctx* ctx, int32_t* config);
 int wlc_set_launch_config(wlc_ctx* ctx, int32_t a_variant, int32_t solve_threads, int32_t xy_threads,
                           int32_t xy_variant);

@@ -1044,7 +1044,7 @@ extern "C" int wlc_iterate(wlc_ctx* c, const wlc_mix_params* mp, double* err, in
 // ------------------------------------------------------------ launch autotuning
 // Candidate launch configurations give bit-identical results (the solve
 // split only changes which thread owns which degree block / m system, and
-// both pass-A variants compute the same sums), so the tuner times them on
+// all variants of passes A and C compute the same sums), so the tuner times them on
 // the instance's own data and keeps the fastest.
 template <typename T> static int autotune_impl(wlc_ctx* c) {
     int rc;
@@ -1056,14 +1056,11 @@ template <typename T> static int autotune_impl(wlc_ctx* c) {
     auto at = [&](int q) -> T* { return c->K ? qf_ring<T>(c, q) : (T*)c->qf + (size_t)q * sl; };
     const StepKind k = fwd_kind(c, s);
     float best = 1e30f;
-    int best_a = c->a_variant, best_t = c->solve_threads, best_x = c->xy_threads, best_z = c->xy_z;
+    int best_t = c->solve_threads, best_x = c->xy_threads, best_z = c->xy_z;
     const bool ms = std::fabs(c->p.nmu) >= 1.0e-5 && c->have_mop;
     for (int xz : {0, 1, 2, 3})
     for (int xt : {256, 512})
-    for (int av : {1, 2}) {
-        if (av == 2 && sizeof(T) != 4) continue;
         for (int th : solve_thread_candidates(c->N)) {
-            c->a_variant = av;
             c->solve_threads = th;
             c->xy_threads = xt;
             c->xy_z = xz;
@@ -1078,14 +1075,12 @@ template <typename T> static int autotune_impl(wlc_ctx* c) {
             CK(cudaGetLastError());
             if (ms_t < best) {
                 best = ms_t;
-                best_a = av;
                 best_t = th;
                 best_x = xt;
                 best_z = xz;
             }
         }
-    }
-    c->a_variant = best_a;
+    c->a_variant = 1;
     c->solve_threads = best_t;
     c->xy_threads = best_x;
     c->xy_z = best_z;

@@ -22,7 +22,7 @@ struct wlc_batch {
         StepArgs<float>* dstep = nullptr;  // [2 directions][nmax + 1][count]
         SolveArgs<float>* dsolve = nullptr;
         size_t smem = 0;
-        int a_variant = 0, solve_threads = 0, xy_threads = 0, xy_z = 0;
+        int solve_threads = 0, xy_threads = 0, xy_z = 0;
         std::vector<int> streamed;              // members with streamed densities
         SliceBatchArgs<float>* dslice = nullptr;  // [streamed]
         bool any_s = false;
@@ -187,7 +187,6 @@ static int batch_issue_group(wlc_batch* b, wlc_batch::Group& g, cudaStream_t st)
         bl.nkx = g.N / 2 + 1;
         bl.lmax = b->inst[g.idx[0]]->L;
         bl.solve_smem = g.smem;
-        bl.a_variant = g.a_variant;
         bl.solve_threads = g.solve_threads;
         bl.xy_threads = g.xy_threads;
         bl.xy_z = g.xy_z;
@@ -395,10 +394,9 @@ extern "C" int wlc_batch_autotune(wlc_batch* b, int32_t* config) {
         auto& g = b->groups[gi];
         const int cnt = (int)g.idx.size();
         float best = 1e30f;
-        int best_a = g.a_variant, best_t = g.solve_threads, best_x = g.xy_threads, best_z = g.xy_z;
+        int best_t = g.solve_threads, best_x = g.xy_threads, best_z = g.xy_z;
         for (int xz : {0, 1, 2, 3})
         for (int xt : {256, 512})
-        for (int av : {1, 2})
             for (int th : solve_thread_candidates(g.N)) {
                 BatchLaunch<float> bl;
                 const size_t e = (size_t)nmax * cnt;  // direction 0, step nmax
@@ -409,7 +407,6 @@ extern "C" int wlc_batch_autotune(wlc_batch* b, int32_t* config) {
                 bl.nkx = g.N / 2 + 1;
                 bl.lmax = b->inst[g.idx[0]]->L;
                 bl.solve_smem = g.smem;
-                bl.a_variant = av;
                 bl.solve_threads = th;
                 bl.xy_threads = xt;
                 bl.xy_z = xz;
@@ -427,19 +424,17 @@ extern "C" int wlc_batch_autotune(wlc_batch* b, int32_t* config) {
                 BCK(cudaGetLastError());
                 if (t < best) {
                     best = t;
-                    best_a = av;
                     best_t = th;
                     best_x = xt;
                     best_z = xz;
                 }
             }
-        g.a_variant = best_a;
         g.solve_threads = best_t;
         g.xy_threads = best_x;
         g.xy_z = best_z;
         if (config) {
             config[5 * gi] = g.N;
-            config[5 * gi + 1] = best_a;
+            config[5 * gi + 1] = 1;
             config[5 * gi + 2] = best_t;
             config[5 * gi + 3] = best_x;
             config[5 * gi + 4] = best_z;

@@ -181,7 +181,6 @@ template <typename T>
 inline StepLaunch<T> make_launch(wlc_ctx* c, StepKind k, const T* h1, const T* h2, const T* h3, T* qout) {
     using C = typename cvec<T>::t;
     StepLaunch<T> L;
-    L.a_variant = c->a_variant;
     L.solve_threads = c->solve_threads;
     L.xy_threads = c->xy_threads;
     L.xy_z = c->xy_z;

@@ -11,6 +11,7 @@
 // the shared column (line stride N+1, conflict free).  Tridiagonal
 // pivots come from a per-(order, block) table keyed by ix^2+iy^2+iz^2 when
 // the grid spacing is isotropic.
+#include <algorithm>
 #include <cstdio>
 
 #include "wlc_attr.h"
@@ -602,11 +603,33 @@ template <typename T> size_t solve_smem_bytes(const SolveArgs<T>& a) {
 
 // Work split of the solve: greedy balance of the degree blocks over P parts
 // and of the m systems over 2P.  threads = N P as the tuner counts them (0:
-// the default); the CTA has 2 N P threads.
-template <typename T> static int solve_parts(int N, int threads) {
+// by the rule below); the CTA has 2 N P threads.
+//
+// Rule: as many parts as still leave few waves.  A CTA's time is about 0.65
+// (loads, FFTs) + the largest part's share of the solve; the columns of the
+// launch come in waves of the CTAs that fit the SMs (shared memory; 80
+// registers a thread in FP32, 128 in FP64).  The estimate names the measured
+// best split, or one within 8 % of it, for N = 16..128 in both precisions;
+// one fixed thread count cost up to 2.2x (FP64 24^3, L = 5: 4 waves, 150 us;
+// 3 parts, one wave: 67 us).
+template <typename T> static int solve_parts(int N, int L, int threads, size_t smem, int columns) {
     const int pmax = kSolveThreads / N < 1 ? 1 : kSolveThreads / N;
-    const int want = threads > 0 ? threads / N : (sizeof(T) == 4 ? 128 : 256) / N;
-    return want < 1 ? 1 : want > pmax ? pmax : want;
+    if (threads > 0) return std::min(std::max(threads / N, 1), pmax);
+    const int fit_smem = std::max(1, (int)(227 * 1024 / (smem + 1024)));
+    const float total = (L + 1) * (L * (2 * L + 1) / 6.0f + 1.5f * L + 1.0f), top = (float)(L * L + 3 * L + 1);
+    int best = 1;
+    float tbest = 1e30f;
+    for (int p = 1; p <= std::min(pmax, L + 1); ++p) {
+        const int warps = (2 * N * p + 31) / 32;
+        const int fit = std::max(1, std::min(fit_smem, (sizeof(T) == 4 ? 25 : 16) / warps));
+        const int waves = (columns + 152 * fit - 1) / (152 * fit);
+        const float t = (float)waves * (0.65f + std::max(1.0f / p, top / total) + 0.01f * p);
+        if (t < tbest) {
+            tbest = t;
+            best = p;
+        }
+    }
+    return best;
 }
 static SolveSplit solve_split(int L, int parts) {
     SolveSplit s{};
@@ -627,8 +650,9 @@ static SolveSplit solve_split(int L, int parts) {
 
 template <typename T, int N> static cudaError_t launch_solve_n(const SolveArgs<T>& a, cudaStream_t st, int threads) {
     if (const cudaError_t e = smem_attr_once((const void*)zfft_solve<T, N>, 227 * 1024); e != cudaSuccess) return e;
-    const int parts = solve_parts<T>(N, threads);
-    zfft_solve<T, N><<<a.nkx * N, 2 * N * parts, solve_smem_bytes<T>(a), st>>>(a, nullptr, solve_split(a.tab.L, parts));
+    const size_t smem = solve_smem_bytes<T>(a);
+    const int parts = solve_parts<T>(N, a.tab.L, threads, smem, a.nkx * N);
+    zfft_solve<T, N><<<a.nkx * N, 2 * N * parts, smem, st>>>(a, nullptr, solve_split(a.tab.L, parts));
     return cudaGetLastError();
 }
 
@@ -650,7 +674,7 @@ template <int N> static cudaError_t set_solve_batched_attr() {
 
 template <int N> static cudaError_t launch_solve_batched_n(const BatchLaunch<float>& b, cudaStream_t st) {
     if (const cudaError_t e = set_solve_batched_attr<N>(); e != cudaSuccess) return e;
-    const int parts = solve_parts<float>(N, b.solve_threads);
+    const int parts = solve_parts<float>(N, b.lmax, b.solve_threads, b.solve_smem, b.nkx * N * b.count);
     zfft_solve<float, N, true><<<dim3(b.nkx * N, 1, b.count), 2 * N * parts, b.solve_smem, st>>>(
         SolveArgs<float>{}, b.dsolve, solve_split(b.lmax, parts));
     return cudaGetLastError();

@@ -16,8 +16,7 @@ __device__ __forceinline__ int fold_idx(int i, int n) { return i <= n / 2 ? i : 
 // MDE_ABC.f90:245-375): order 1 (1 - ds w) q1; order 2
 // 2 q1 - q2/2 - ds w (2 q1 - q2); order 3 sum_j c_j(r) q_j with
 // c = (3 - 3 ds w, -3/2 + 3 ds w, 1/3 - ds w) precomputed per block.
-// FP32 form shared by both pass-A kernels (so that they give identical
-// results): dw = ds w(r) rounded once, every operation rounded explicitly.
+// FP32 form (the same for every launch variant): dw = ds w(r) rounded once, every operation rounded explicitly.
 // Split-scheme steps (kSplitOrder) pass e^{-w ds/2} as dw: q1 e^{-w ds/2}.
 __device__ __forceinline__ float rhs_f32(int order, float q1, float q2, float q3, float dw, float third) {
     if (order == 0) return q1;
@@ -247,84 +246,6 @@ __global__ void __launch_bounds__(512) rhs_fft_xy(StepArgs<T> a0, const StepArgs
     store_phat<T, N, Z>(a, out, i, z0);
 }
 
-// FP32 pass A with the history planes staged by cp.async, double-buffered
-// across the CTA's z planes (plane zz+1 in flight while zz is transformed).
-template <int N> struct StagedA {
-    static constexpr int Z = zg_planes(N, 4);
-    static constexpr size_t P = (size_t)N * N;
-    static constexpr size_t bytes = 8 * ((size_t)N + (size_t)xplane(N) + (size_t)Z * N * (N / 2 + 1)) + 2 * 4 * P * 4;
-    static constexpr bool fits = bytes <= 220 * 1024;
-};
-
-__device__ __forceinline__ float rhs_staged(const float* st, int order, size_t P, size_t idx, float third) {
-    const float q1 = st[idx];
-    if (order == 0) return q1;
-    if (order == 1 || order == kSplitOrder) return rhs_f32(order, q1, 0.0f, 0.0f, st[P + idx], third);
-    if (order == 2) return rhs_f32(2, q1, st[P + idx], 0.0f, st[2 * P + idx], third);
-    return rhs_f32(3, q1, st[P + idx], st[2 * P + idx], st[3 * P + idx], third);
-}
-
-template <int N, bool B = false>
-__global__ void __launch_bounds__(512) rhs_fft_xy_staged(StepArgs<float> a0, const StepArgs<float>* __restrict__ batch) {
-    const StepArgs<float> a = pick_args<B>(a0, batch);
-    using C = float2;
-    constexpr int Z = StagedA<N>::Z;
-    constexpr int NKX = N / 2 + 1;
-    constexpr int NR = N * N * N;
-    constexpr size_t P = StagedA<N>::P;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    C* tw = reinterpret_cast<C*>(smem_raw);
-    C* zb = tw + N;                   // packed row pairs, row stride xrow(N)
-    C* out = zb + xplane(N);
-    float* stage = reinterpret_cast<float*>(out + (size_t)Z * N * NKX);  // [2][4][P]
-    const int i = blockIdx.y;
-    const int z0 = blockIdx.x * Z;
-    const int order = a.order;
-    const float* src[4];
-    int ns = 0;
-    src[ns++] = a.h1 + (size_t)i * NR;
-    if (hist_slices(order) >= 2) src[ns++] = a.h2 + (size_t)i * NR;
-    if (hist_slices(order) >= 3) src[ns++] = a.h3 + (size_t)i * NR;
-    if (order >= 1) src[ns++] = a.dsw;
-    auto issue = [&](int zz, int buf) {
-        const size_t zoff = (size_t)(z0 + zz) * P;
-        for (int q = 0; q < ns; ++q) {
-            const float* g = src[q] + zoff;
-            float* d = stage + ((size_t)buf * 4 + q) * P;
-            for (size_t e = (size_t)threadIdx.x * 4; e < P; e += (size_t)blockDim.x * 4) cp_async16(d + e, g + e);
-        }
-        cp_async_commit();
-    };
-    for (int e = threadIdx.x; e < N; e += blockDim.x) tw[e] = a.twg[e];
-    issue(0, 0);
-    for (int zz = 0; zz < Z; ++zz) {
-        if (zz + 1 < Z) {
-            issue(zz + 1, (zz + 1) & 1);
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
-        __syncthreads();
-        const float* st = stage + (size_t)(zz & 1) * 4 * P;
-        const size_t zoff = (size_t)(z0 + zz) * P;
-        for (int e = threadIdx.x; e < (N / 2) * N; e += blockDim.x) {
-            const int p = e / N, x = e % N;
-            const size_t ia = (size_t)(2 * p) * N + x, ib = ia + N;
-            float va = rhs_staged(st, order, P, ia, a.third);
-            float vb = rhs_staged(st, order, P, ib, a.third);
-            if (a.msterm) {
-                va += a.msterm[(size_t)i * NR + zoff + ia];
-                vb += a.msterm[(size_t)i * NR + zoff + ib];
-            }
-            zb[p * xrow(N) + x] = make_float2(va, vb);
-        }
-        __syncthreads();
-        fwd_x_planes<float, N, Z, 1>(zb, out, zz, tw);
-    }
-    y_planes<float, N, Z, -1>(out, tw);
-    store_phat<float, N, Z>(a, out, i, z0);
-}
-
 // ---------------------------------------------------------------- pass C
 __host__ __device__ constexpr int ilog2(int n) { return n > 1 ? 1 + ilog2(n / 2) : 0; }
 // what the y-FFTs of pass C leave: fixed-point numbers in the FP64 form
@@ -469,19 +390,28 @@ template <typename T, int N, bool B> static cudaError_t set_xy_attrs() {
         set((const void*)rhs_fft_xy<T, N, B, 3>, big);
         set((const void*)ifft_xy<T, N, B, 3>, big);
     }
-    if constexpr (sizeof(T) == 4 && StagedA<N>::fits) set((const void*)rhs_fft_xy_staged<N, B>, (int)StagedA<N>::bytes);
     return e;
 }
 
-// threads per CTA of the generic pass A and of pass C: 256 (default) or 512
-static inline int xy_block(int threads) { return threads == 512 ? 512 : 256; }
-
-// pass A variant: 0 = default (staged where it fits), 1 = generic, 2 = staged
-template <typename T, int N> static bool use_staged(int variant) {
-    if constexpr (sizeof(T) == 4 && StagedA<N>::fits)
-        return variant != 1;
-    else
-        return false;
+// Launch shape of passes A and C when none is set (threads = variant = 0),
+// by the CTAs that fit an SM's shared memory.  FP32: the batched x-FFTs on
+// half planes (variant 3: fewest barriers and still several CTAs), unless
+// that leaves one CTA; 256 threads from 4 CTAs on, else 512.  FP64: whole
+// planes with batched x-FFTs while 4 CTAs fit (twice the work per barrier),
+// else half planes; 512 threads for a lone CTA.  Measured per step (us,
+// 256-thread variant 0 -> this): FP32 pass A 24^3 16 -> 14, 48^3 70 -> 56,
+// 64^3 189 -> 171, 128^3 3570 -> 2650; pass C 64^3 135 -> 109, 128^3 1956 ->
+// 1695; FP64 pass A 40^3 120 -> 112, 64^3 655 -> 527, pass C 24^3 22 -> 15.
+template <typename T> static void xy_shape(int N, int& threads, int& variant) {
+    if (threads == 0 && variant == 0) {
+        auto ctas = [&](int v) { return (int)(227 * 1024 / (smem_xy<T>(N, v) + 1024)); };
+        if (sizeof(T) == 4)
+            variant = ctas(3) >= 2 ? 3 : 1;
+        else
+            variant = ctas(2) >= 4 ? 2 : 1;
+        threads = ctas(variant) >= (sizeof(T) == 4 ? 4 : 2) ? 256 : 512;
+    }
+    threads = threads == 512 ? 512 : 256;
 }
 
 // generic pass A / pass C launches in variant V (bit 0 half planes, bit 1
@@ -493,14 +423,15 @@ static void launch_xy(bool do_a, const StepArgs<T>& a, const StepArgs<T>* batch,
     const size_t sxy = smem_xy<T>(N, V);
     const dim3 g(N / Z, M, count);
     if (do_a)
-        rhs_fft_xy<T, N, B, V><<<g, xy_block(threads), sxy, st>>>(a, batch);
+        rhs_fft_xy<T, N, B, V><<<g, threads, sxy, st>>>(a, batch);
     else
-        ifft_xy<T, N, B, V><<<g, xy_block(threads), sxy, st>>>(a, batch);
+        ifft_xy<T, N, B, V><<<g, threads, sxy, st>>>(a, batch);
 }
 
 template <typename T, int N, bool B>
 static void launch_xy_any(int variant, bool do_a, const StepArgs<T>& a, const StepArgs<T>* batch, int M, int count,
                           int threads, cudaStream_t st) {
+    xy_shape<T>(N, threads, variant);
     if ((variant & 2) && smem_xy<T>(N, variant) > 200 * 1024) variant &= 1;  // batched x-FFTs do not fit
     switch (variant & 3) {
         case 1: launch_xy<T, N, B, 1>(do_a, a, batch, M, count, threads, st); break;
@@ -511,18 +442,9 @@ static void launch_xy_any(int variant, bool do_a, const StepArgs<T>& a, const St
 }
 
 template <typename T, int N> static cudaError_t launch_n(const StepLaunch<T>& s, cudaStream_t st) {
-    constexpr int Z = zg_planes(N, sizeof(T));
     if (const cudaError_t ea = set_xy_attrs<T, N, false>(); ea != cudaSuccess) return ea;
-    const dim3 gxy(N / Z, s.step.M);
     if (s.events) cudaEventRecord(s.events[0], st);
-    if (s.do_a) {
-        bool staged = false;
-        if constexpr (sizeof(T) == 4 && StagedA<N>::fits) {
-            staged = use_staged<T, N>(s.a_variant);
-            if (staged) rhs_fft_xy_staged<N><<<gxy, 512, StagedA<N>::bytes, st>>>(s.step, nullptr);
-        }
-        if (!staged) launch_xy_any<T, N, false>(s.xy_z, true, s.step, nullptr, s.step.M, 1, s.xy_threads, st);
-    }
+    if (s.do_a) launch_xy_any<T, N, false>(s.xy_z, true, s.step, nullptr, s.step.M, 1, s.xy_threads, st);
     if (s.events) cudaEventRecord(s.events[1], st);
     if (s.do_b) launch_solve<T>(N, s.solve, st, s.solve_threads);
     if (s.events) cudaEventRecord(s.events[2], st);
@@ -532,15 +454,8 @@ template <typename T, int N> static cudaError_t launch_n(const StepLaunch<T>& s,
 }
 
 template <int N> static cudaError_t launch_batched_n(const BatchLaunch<float>& b, cudaStream_t st) {
-    constexpr int Z = zg_planes(N, 4);
     if (const cudaError_t ea = set_xy_attrs<float, N, true>(); ea != cudaSuccess) return ea;
-    const dim3 gxy(N / Z, b.M, b.count);
-    bool staged = false;
-    if constexpr (StagedA<N>::fits) {
-        staged = use_staged<float, N>(b.a_variant);
-        if (staged) rhs_fft_xy_staged<N, true><<<gxy, 512, StagedA<N>::bytes, st>>>(StepArgs<float>{}, b.dstep);
-    }
-    if (!staged) launch_xy_any<float, N, true>(b.xy_z, true, StepArgs<float>{}, b.dstep, b.M, b.count, b.xy_threads, st);
+    launch_xy_any<float, N, true>(b.xy_z, true, StepArgs<float>{}, b.dstep, b.M, b.count, b.xy_threads, st);
     cudaError_t e = launch_solve_batched(N, b, st);
     if (e != cudaSuccess) return e;
     launch_xy_any<float, N, true>(b.xy_z, false, StepArgs<float>{}, b.dstep, b.M, b.count, b.xy_threads, st);
