@@ -304,6 +304,92 @@ template <typename T> static int use_precision(wlc_ctx* c) {
     return WLC_OK;
 }
 
+// the coupling lists of the Theta term and of the orientation tensor
+static int build_class_lists(wlc_ctx* c) {
+    const int M = c->M;
+    struct Host {
+        std::vector<uint16_t> ptr{0}, gptr{0};
+        std::vector<int16_t> col, gcol, order;
+        std::vector<double> val, gval;
+    };
+    auto finish = [&](Host& h, ClassLists& d) -> int {
+        d.n = (int)h.val.size();
+        d.ng = (int)h.gcol.size();
+        for (int a = 0; a < 5; ++a) {
+            d.vmin[a] = 1e300;
+            d.vmax[a] = 0.0;
+        }
+        for (int i = 0; i < M; ++i)
+            for (int a = 0; a < 5; ++a)
+                for (int e = h.ptr[5 * i + a]; e < h.ptr[5 * i + a + 1]; ++e) {
+                    d.vmin[a] = std::min(d.vmin[a], std::fabs(h.val[e]));
+                    d.vmax[a] = std::max(d.vmax[a], std::fabs(h.val[e]));
+                }
+        for (int i = 0; i < M; ++i) h.order.push_back((int16_t)i);
+        std::stable_sort(h.order.begin(), h.order.end(), [&](int16_t a, int16_t b) {
+            return h.ptr[5 * a + 5] - h.ptr[5 * a] > h.ptr[5 * b + 5] - h.ptr[5 * b];
+        });
+        int rc;
+        uint16_t* pu;
+        int16_t* pi;
+        double* pd;
+        if ((rc = upload(c, &pu, h.ptr))) return rc;
+        d.ptr = pu;
+        if ((rc = upload(c, &pu, h.gptr))) return rc;
+        d.gptr = pu;
+        if ((rc = upload(c, &pi, h.col))) return rc;
+        d.col = pi;
+        if ((rc = upload(c, &pi, h.gcol))) return rc;
+        d.gcol = pi;
+        if ((rc = upload(c, &pi, h.order))) return rc;
+        d.order = pi;
+        if ((rc = upload(c, &pd, h.val))) return rc;
+        d.val = pd;
+        if ((rc = upload(c, &pd, h.gval))) return rc;
+        d.gval = pd;
+        return WLC_OK;
+    };
+    // J in the thresholded form of the reference's sparse lists
+    std::vector<double> J[5];
+    for (int a = 0; a < 5; ++a) {
+        J[a].assign((size_t)M * M, 0.0);
+        for (size_t e = 0; e < c->tab.Jsp[a].size(); ++e)
+            J[a][(size_t)c->tab.Jsp[a].row[e] * M + c->tab.Jsp[a].col[e]] = c->tab.Jsp[a].val[e];
+    }
+    Host th, jh;
+    for (int i = 0; i < M; ++i) {
+        for (int a = 0; a < 5; ++a) {
+            for (int j = 0; j < M; ++j) {
+                const size_t o = (size_t)i * M + j;
+                int nz = 0;
+                for (int q = 0; q < 5; ++q) nz += c->tab.T[q][o] != 0.0;
+                if (nz == 1 && c->tab.T[a][o] != 0.0) {
+                    th.col.push_back((int16_t)j);
+                    th.val.push_back(c->tab.T[a][o]);
+                }
+                if (nz > 1 && a == 0) {
+                    th.gcol.push_back((int16_t)j);
+                    for (int q = 0; q < 5; ++q) th.gval.push_back(c->tab.T[q][o]);
+                }
+                const double v = a == 0   ? 0.5 * (J[0][o] + J[1][o])
+                                 : a == 1 ? 0.5 * (J[0][o] - J[1][o])
+                                          : J[a][o];
+                if (v != 0.0) {
+                    jh.col.push_back((int16_t)j);
+                    jh.val.push_back(v);
+                }
+            }
+            th.ptr.push_back((uint16_t)th.val.size());
+            jh.ptr.push_back((uint16_t)jh.val.size());
+        }
+        th.gptr.push_back((uint16_t)th.gcol.size());
+        jh.gptr.push_back(0);
+    }
+    int rc;
+    if ((rc = finish(th, c->thl))) return rc;
+    return finish(jh, c->jl);
+}
+
 int create_impl(const wlc_params* p, cudaStream_t ext, wlc_ctx** out) {
     if (!p || !out) return WLC_E_PARAM;
     *out = nullptr;
@@ -349,57 +435,7 @@ int create_impl(const wlc_params* p, cudaStream_t ext, wlc_ctx** out) {
         }
     }
     apply_box(c);
-    // Theta and J lists
-    {
-        std::vector<int16_t> tr, tcol;
-        std::vector<double> tv;
-        const int M = c->M;
-        for (int i = 0; i < M; ++i)
-            for (int j = 0; j < M; ++j) {
-                bool any = false;
-                for (int a = 0; a < 5; ++a) any = any || c->tab.T[a][(size_t)i * M + j] != 0.0;
-                if (!any) continue;
-                tr.push_back((int16_t)i);
-                tcol.push_back((int16_t)j);
-                for (int a = 0; a < 5; ++a) tv.push_back(c->tab.T[a][(size_t)i * M + j]);
-            }
-        int16_t* p16;
-        double* pd;
-        if ((rc = upload(c, &p16, tr))) return rc;
-        c->thl.row = p16;
-        if ((rc = upload(c, &p16, tcol))) return rc;
-        c->thl.col = p16;
-        if ((rc = upload(c, &pd, tv))) return rc;
-        c->thl.val = pd;
-        c->thl.n = (int)tr.size();
-        std::vector<int> rp(M + 1, 0);  // entries are emitted row by row
-        for (int16_t i : tr) rp[i + 1]++;
-        for (int i = 0; i < M; ++i) rp[i + 1] += rp[i];
-        int* pr;
-        if ((rc = upload(c, &pr, rp))) return rc;
-        c->thl.rowptr = pr;
-        std::vector<int> jp(6, 0);
-        std::vector<int16_t> jr, jc;
-        std::vector<double> jv;
-        for (int a = 0; a < 5; ++a) {
-            for (size_t e = 0; e < c->tab.Jsp[a].size(); ++e) {
-                jr.push_back((int16_t)c->tab.Jsp[a].row[e]);
-                jc.push_back((int16_t)c->tab.Jsp[a].col[e]);
-                jv.push_back(c->tab.Jsp[a].val[e]);
-            }
-            jp[a + 1] = (int)jv.size();
-        }
-        int* pi;
-        if ((rc = upload(c, &pi, jp))) return rc;
-        c->jl.ptr = pi;
-        if ((rc = upload(c, &p16, jr))) return rc;
-        c->jl.row = p16;
-        if ((rc = upload(c, &p16, jc))) return rc;
-        c->jl.col = p16;
-        if ((rc = upload(c, &pd, jv))) return rc;
-        c->jl.val = pd;
-        c->jl.n = (int)jv.size();
-    }
+    if ((rc = build_class_lists(c))) return rc;
     c->nkeys = 3 * (c->N / 2) * (c->N / 2) + 1;
     c->npiv = (c->L + 1) * (c->L + 2) / 2;
     if ((rc = c->fp32 ? alloc_fields<float>(c) : alloc_fields<double>(c))) return rc;

@@ -198,7 +198,7 @@ static int batch_issue_group(wlc_batch* b, wlc_batch::Group& g, cudaStream_t st)
     auto slices = [&](int s) {
         if (g.streamed.empty()) return;
         const wlc_ctx* c0 = b->inst[g.streamed[0]];
-        launch_density_slice_batched<float>(g.dslice, (int)g.streamed.size(), c0->nr, s, b->M, c0->jl.n,
+        launch_density_slice_batched<float>(g.dslice, (int)g.streamed.size(), c0->nr, s, b->M, c0->jl,
                                             g.any_s ? 1 : 0, st);
         b->launches++;
     };

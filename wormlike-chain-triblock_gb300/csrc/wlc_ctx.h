@@ -41,8 +41,7 @@ struct wlc_ctx {
     std::vector<void*> allocs;
     SolveTablesT<double> sd{};
     SolveTablesT<float> sf{};
-    ThetaLists thl{};
-    JLists jl{};
+    ClassLists thl{}, jl{};
     void* twg = nullptr;
     // per-precision operator data ([0] FP64, [1] FP32); twg / pivtab /
     // have_piv above alias the active one

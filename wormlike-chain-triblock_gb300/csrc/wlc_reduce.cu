@@ -111,312 +111,493 @@ template <typename T> __device__ __forceinline__ void vstore(T* p, const T* v) {
     *reinterpret_cast<typename VecOf<T>::t*>(p) = x;
 }
 
-// shared-memory layout of ms_term: hc[M][TILE] (16-byte aligned rows) | val[5n] | rowptr[M+1] | col[n]
-template <typename T> __host__ __device__ inline size_t ms_smem_bytes(int n, int M) {
-    return sizeof(T) * ((size_t)5 * n + (size_t)M * PointTile<T>::value) + sizeof(int) * (size_t)(M + 1) +
-           sizeof(int16_t) * (size_t)n;
+// ------------------------------------------------------------ coupling lists
+// The per-point kernels below (Theta term, orientation tensor) are sparse
+// products with the coefficient vector of every grid point.  One CTA stages
+// the lists once and walks tiles of TILE points; a thread takes P points (one
+// 16-byte vector) and every kGroups-th row, longest rows first, so that one
+// list entry (two broadcast reads) and one 16-byte read of the tile serve P
+// points.  A component's entries of a row are summed before the point's
+// factor is applied: one multiply-add per entry and point.
+constexpr int kGroups = 16;
+template <typename T> struct Pts {
+    static constexpr int P = 16 / sizeof(T), LANES = PointTile<T>::value / P, THREADS = LANES * kGroups;
+};
+
+template <typename T> struct ListSmem {
+    T *val, *gval;
+    uint16_t *ptr, *gptr;
+    int16_t *col, *gcol, *order;
+};
+template <typename T> __host__ __device__ inline size_t list_bytes(int n, int ng, int M) {
+    return sizeof(T) * ((size_t)n + 5 * ng) + 2 * ((size_t)5 * M + 1 + M + 1 + n + ng + M);
+}
+template <typename T> __device__ __forceinline__ ListSmem<T> stage_lists(const ClassLists& l, int M, void* at) {
+    ListSmem<T> m;
+    m.val = reinterpret_cast<T*>(at);
+    m.gval = m.val + l.n;
+    m.ptr = reinterpret_cast<uint16_t*>(m.gval + 5 * l.ng);
+    m.gptr = m.ptr + 5 * M + 1;
+    m.col = reinterpret_cast<int16_t*>(m.gptr + M + 1);
+    m.gcol = m.col + l.n;
+    m.order = m.gcol + l.ng;
+    for (int e = threadIdx.x; e < l.n; e += blockDim.x) {
+        m.val[e] = (T)l.val[e];
+        m.col[e] = l.col[e];
+    }
+    for (int e = threadIdx.x; e < 5 * l.ng; e += blockDim.x) m.gval[e] = (T)l.gval[e];
+    for (int e = threadIdx.x; e < l.ng; e += blockDim.x) m.gcol[e] = l.gcol[e];
+    for (int e = threadIdx.x; e <= 5 * M; e += blockDim.x) m.ptr[e] = l.ptr[e];
+    for (int e = threadIdx.x; e <= M; e += blockDim.x) m.gptr[e] = l.gptr[e];
+    for (int e = threadIdx.x; e < M; e += blockDim.x) m.order[e] = l.order[e];
+    return m;
 }
 
-// The Theta lists (values converted to the compute type) are staged once per
-// CTA; the CTA then walks tiles of TILE points.  Thread (k, g) handles point
-// k of the tile and rows i = g, g + kMsGroups, ... of its output.
+// sum of the entries [e0, e1) times the tile's coefficients, at P points
 template <typename T>
-__global__ void __launch_bounds__(PointTile<T>::value * kMsGroups)
+__device__ __forceinline__ void gather_sum(const ListSmem<T>& m, int e0, int e1, const T* tile, T* y) {
+    constexpr int P = Pts<T>::P, TILE = PointTile<T>::value;
+#pragma unroll
+    for (int u = 0; u < P; ++u) y[u] = (T)0;
+#pragma unroll 2
+    for (int e = e0; e < e1; ++e) {
+        const T v = m.val[e];
+        T h[P];
+        vload<T>(tile + m.col[e] * TILE, h);
+#pragma unroll
+        for (int u = 0; u < P; ++u) y[u] = fma(v, h[u], y[u]);
+    }
+}
+
+// shared-memory layout of ms_term: hc[M][TILE] | coef[5][TILE] | lists
+template <typename T> __host__ __device__ inline size_t ms_smem_bytes(const ClassLists& tl, int M) {
+    return sizeof(T) * (size_t)(M + 5) * PointTile<T>::value + list_bytes<T>(tl.n, tl.ng, M);
+}
+
+// Bound by the shared-memory reads of the tile (one 16-byte read per entry and
+// P points).  128^3, L = 12 in FP32: 6.1 ms a launch with one point a thread
+// and all five components of every entry, 2.5 ms in this form.
+template <typename T>
+__global__ void __launch_bounds__(Pts<T>::THREADS)
     ms_term(const T* __restrict__ h1, const T* __restrict__ h2, const T* __restrict__ h3, int order,
-            const double* __restrict__ mop, ThetaLists tl, double ds, double thresh, int M, int64_t nr,
+            const double* __restrict__ mop, ClassLists tl, double ds, double thresh, int M, int64_t nr,
             T* __restrict__ out) {
-    constexpr int TILE = PointTile<T>::value;
+    constexpr int TILE = PointTile<T>::value, P = Pts<T>::P;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* hc = reinterpret_cast<T*>(smem_raw);  // [M][TILE]: BDF history combination of the tile's points
-    T* sval = hc + (size_t)M * TILE;
-    int* srp = reinterpret_cast<int*>(sval + (size_t)5 * tl.n);
-    int16_t* scol = reinterpret_cast<int16_t*>(srp + M + 1);
-    for (int e = threadIdx.x; e < 5 * tl.n; e += blockDim.x) sval[e] = (T)tl.val[e];
-    for (int e = threadIdx.x; e <= M; e += blockDim.x) srp[e] = tl.rowptr[e];
-    for (int e = threadIdx.x; e < tl.n; e += blockDim.x) scol[e] = tl.col[e];
-    const int k = threadIdx.x % TILE, g = threadIdx.x / TILE;
+    T* sco = hc + (size_t)M * TILE;          // [5][TILE]: factors of the components
+    const ListSmem<T> m = stage_lists<T>(tl, M, sco + 5 * TILE);
+    const int k = (threadIdx.x % Pts<T>::LANES) * P, g = threadIdx.x / Pts<T>::LANES;
     const T th_min = (T)thresh;
     for (int64_t r0 = (int64_t)blockIdx.x * TILE; r0 < nr; r0 += (int64_t)gridDim.x * TILE) {
-        __syncthreads();  // tables staged / previous tile consumed
-        // 16-byte vectors of V consecutive points (nr and r0 are multiples of V)
-        constexpr int V = 16 / sizeof(T);
-        using VT = typename VecOf<T>::t;
-        for (int idx = threadIdx.x; idx < M * (TILE / V); idx += blockDim.x) {
-            const int j = idx / (TILE / V), kk = (idx % (TILE / V)) * V;
-            const int64_t r = r0 + kk;
-            T v[V] = {};
-            if (r < nr) {
-                const int64_t o = (int64_t)j * nr + r;
-                T q1[V], q2[V], q3[V];
-                vload<T>(h1 + o, q1);
-                if (order >= 2) vload<T>(h2 + o, q2);
-                if (order >= 3) vload<T>(h3 + o, q3);
+        __syncthreads();  // lists staged / previous tile consumed
+        for (int idx = threadIdx.x; idx < M * (TILE / P); idx += blockDim.x) {
+            const int j = idx / (TILE / P), kk = (idx % (TILE / P)) * P;
+            const int64_t o = (int64_t)j * nr + r0 + kk;  // nr is a multiple of TILE
+            T v[P], q1[P], q2[P], q3[P];
+            vload<T>(h1 + o, q1);
+            if (order >= 2) vload<T>(h2 + o, q2);
+            if (order >= 3) vload<T>(h3 + o, q3);
 #pragma unroll
-                for (int u = 0; u < V; ++u) {
-                    if (order == 1)
-                        v[u] = q1[u];
-                    else if (order == 2)
-                        v[u] = (T)2 * q1[u] - q2[u];
-                    else
-                        v[u] = (T)3 * q1[u] - (T)3 * q2[u] + q3[u];
-                }
+            for (int u = 0; u < P; ++u) {
+                if (order == 1)
+                    v[u] = q1[u];
+                else if (order == 2)
+                    v[u] = (T)2 * q1[u] - q2[u];
+                else
+                    v[u] = (T)3 * q1[u] - (T)3 * q2[u] + q3[u];
             }
             vstore<T>(hc + j * TILE + kk, v);
         }
-        (void)sizeof(VT);
-        __syncthreads();
-        const int64_t r = r0 + k;
-        if (r >= nr) continue;
-        // Theta_ij(r) = sum_c coef_c T_c(i,j), entries below the threshold dropped
+        // Theta_ij(r) = sum_c coef_c T_c(i,j)
         // (M01 = mop[0 + 3*1] = M_OP(k,0,1) in Fortran order; the tensor is symmetric)
-        const T coef[5] = {(T)(mop[0 * nr + r] - mop[4 * nr + r]), (T)mop[8 * nr + r], (T)mop[3 * nr + r],
-                           (T)mop[6 * nr + r], (T)mop[7 * nr + r]};
-        const T* hv = hc + k;
-        // entries in groups of four with independent partial sums (the list
-        // loads and the coefficient gathers of four entries overlap)
-        auto term = [&](int e) -> T {
-            const T* v5 = sval + 5 * e;
-            const T th = coef[0] * v5[0] + coef[1] * v5[1] + coef[2] * v5[2] + coef[3] * v5[3] + coef[4] * v5[4];
-            return fabs(th) < th_min ? (T)0 : th * hv[scol[e] * TILE];
-        };
-        for (int i = g; i < M; i += kMsGroups) {
-            T a0 = (T)0, a1 = (T)0, a2 = (T)0, a3 = (T)0;
-            const int e1 = srp[i + 1];
-            int e = srp[i];
-            for (; e + 4 <= e1; e += 4) {
-                a0 += term(e);
-                a1 += term(e + 1);
-                a2 += term(e + 2);
-                a3 += term(e + 3);
+        for (int idx = threadIdx.x; idx < 5 * TILE; idx += blockDim.x) {
+            const int c = idx / TILE;
+            const int64_t r = r0 + idx % TILE;
+            const double v = c == 0   ? mop[r] - mop[4 * nr + r]
+                             : c == 1 ? mop[8 * nr + r]
+                                      : mop[(c == 2 ? 3 : c == 3 ? 6 : 7) * nr + r];
+            sco[idx] = (T)v;
+        }
+        __syncthreads();
+        // entries with |Theta| below the threshold are dropped: none or all of
+        // a component's where its factor is large or tiny enough, else entry
+        // by entry (bit c of mixed)
+        T cf[5][P];
+        unsigned mixed = 0;
+#pragma unroll
+        for (int c = 0; c < 5; ++c) {
+            vload<T>(sco + c * TILE + k, cf[c]);
+#pragma unroll
+            for (int u = 0; u < P; ++u) {
+                const T a = fabs(cf[c][u]);
+                if (a * (T)tl.vmax[c] < th_min * (T)0.5)
+                    cf[c][u] = (T)0;
+                else if (!(a * (T)tl.vmin[c] > th_min * (T)2))
+                    mixed |= 1u << c;
             }
-            for (; e < e1; ++e) a0 += term(e);
-            out[(int64_t)i * nr + r] = (T)ds * ((a0 + a1) + (a2 + a3));
+        }
+        for (int row = g; row < M; row += kGroups) {
+            const int i = m.order[row];
+            const uint16_t* pt = m.ptr + 5 * i;
+            T acc[P] = {};
+            int e0 = pt[0];
+#pragma unroll
+            for (int c = 0; c < 5; ++c) {
+                const int e1 = pt[c + 1];
+                if (!((mixed >> c) & 1u)) {
+                    T y[P];
+                    gather_sum<T>(m, e0, e1, hc + k, y);
+#pragma unroll
+                    for (int u = 0; u < P; ++u) acc[u] = fma(cf[c][u], y[u], acc[u]);
+                } else {
+                    for (int e = e0; e < e1; ++e) {
+                        const T v = m.val[e];
+                        T h[P];
+                        vload<T>(hc + m.col[e] * TILE + k, h);
+#pragma unroll
+                        for (int u = 0; u < P; ++u) {
+                            const T th = cf[c][u] * v;
+                            if (!(fabs(th) < th_min)) acc[u] = fma(th, h[u], acc[u]);
+                        }
+                    }
+                }
+                e0 = e1;
+            }
+            for (int e = m.gptr[i]; e < m.gptr[i + 1]; ++e) {
+                T h[P];
+                vload<T>(hc + m.gcol[e] * TILE + k, h);
+#pragma unroll
+                for (int u = 0; u < P; ++u) {
+                    T th = (T)0;
+#pragma unroll
+                    for (int c = 0; c < 5; ++c) th = fma(sco[c * TILE + k + u], m.gval[5 * e + c], th);
+                    if (!(fabs(th) < th_min)) acc[u] = fma(th, h[u], acc[u]);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < P; ++u) acc[u] *= (T)ds;
+            vstore<T>(out + (int64_t)i * nr + r0 + k, acc);
         }
     }
 }
 
 // ------------------------------------------------------------ densities
+// Running dot products in (at least) FP64 accuracy at P points.  FP32 slices:
+// a product and its error are exact in two floats and are added to a sum of
+// three floats by error-free additions (72 bits; the FP64 pipe has 1/64 of
+// the FP32 rate, and one multiply-add with its two conversions costs 192
+// clocks of a scheduler there against 22 here).
+__device__ __forceinline__ float two_sum(float a, float b, float& err) {
+    const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
+    err = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+    return s;
+}
+template <typename T, int P> struct Dots;
+template <int P> struct Dots<double, P> {
+    static constexpr int W = 1;  // words per point
+    double s[P] = {};
+    __device__ __forceinline__ void add(int u, double a, double b) { s[u] = fma(a, b, s[u]); }
+    __device__ __forceinline__ void put(int u, double* w, int) const { w[0] = s[u]; }
+    __device__ __forceinline__ void merge(int u, const double* w, int) { s[u] += w[0]; }
+    __device__ __forceinline__ double get(int u) const { return s[u]; }
+};
+template <int P> struct Dots<float, P> {
+    static constexpr int W = 3;
+    float s[P] = {}, c[P] = {}, d[P] = {};
+    __device__ __forceinline__ void add3(int u, float p, float e, float f) {
+        float t1, t2, t3;
+        s[u] = two_sum(s[u], p, t1);
+        c[u] = two_sum(c[u], t1, t2);
+        c[u] = two_sum(c[u], e, t3);
+        d[u] = __fadd_rn(d[u], __fadd_rn(__fadd_rn(t2, t3), f));
+    }
+    __device__ __forceinline__ void add(int u, float a, float b) {
+        const float p = __fmul_rn(a, b);
+        add3(u, p, __fmaf_rn(a, b, -p), 0.0f);
+    }
+    __device__ __forceinline__ void put(int u, float* w, int st) const {
+        w[0] = s[u];
+        w[st] = c[u];
+        w[2 * st] = d[u];
+    }
+    __device__ __forceinline__ void merge(int u, const float* w, int st) { add3(u, w[0], w[st], w[2 * st]); }
+    // an overflow leaves a not-a-number in the error terms: the sum itself says which
+    __device__ __forceinline__ double get(int u) const {
+        const double e = (double)c[u] + (double)d[u];
+        return isfinite(s[u]) && isfinite(e) ? (double)s[u] + e : (double)s[u];
+    }
+};
+
 // raw[b][r] = sum_i S1_{s in block b}(q_i q*_i); junc[j][r] = sum_i q_i q*_i at
-// s = NA, NA+NB, Nmax; qend[r] = q_0(r, Nmax).
-// sum_i a[i*stride] c[i*stride] in FP64 with four independent partial sums
-// (more loads in flight per thread; fixed order, so deterministic)
-template <typename T>
-__device__ __forceinline__ double dot_coeffs(const T* __restrict__ a, const T* __restrict__ c, int M, int64_t stride) {
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-    int i = 0;
-    for (; i + 4 <= M; i += 4) {
-        s0 += (double)a[i * stride] * (double)c[i * stride];
-        s1 += (double)a[(i + 1) * stride] * (double)c[(i + 1) * stride];
-        s2 += (double)a[(i + 2) * stride] * (double)c[(i + 2) * stride];
-        s3 += (double)a[(i + 3) * stride] * (double)c[(i + 3) * stride];
-    }
-    for (; i < M; ++i) s0 += (double)a[i * stride] * (double)c[i * stride];
-    return (s0 + s1) + (s2 + s3);
-}
-
-template <typename T>
-__global__ void density_accum(const T* __restrict__ qf, const T* __restrict__ qb, DensityArgs d,
-                              double* __restrict__ raw, double* __restrict__ junc, double* __restrict__ qend) {
-    const int64_t nr = d.nr;
-    const int64_t sl = (int64_t)d.M * nr;
-    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < nr; r += (int64_t)gridDim.x * blockDim.x) {
-        for (int b = 0; b < 3; ++b) {
-            double acc = 0.0;
-            const int s0 = d.nstart[b], n = d.ns[b];
-            if (n > 0) {
-                for (int s = s0; s <= s0 + n; ++s) {
-                    const int j = s - s0;
-                    const double wgt = (j == 0 || j == n) ? 1.0 : ((j & 1) ? 4.0 : 2.0);
-                    const double sum = dot_coeffs(qf + s * sl + r, qb + s * sl + r, d.M, nr);
-                    acc += wgt * sum;
+// s = NA, NA+NB, Nmax; qend[r] = q_0(r, Nmax).  Every slice is read once.  A
+// CTA's threads are G groups of coefficients for 256 / G times P points; the
+// larger G serves grids that would not fill the SMs otherwise.
+// FP32, 64^3, L = 10, 101 slices (25.6 GB): 8.1 ms; with conversions and
+// multiply-adds on the FP64 pipe the iteration took 10.7 ms longer.
+template <typename T, int P, int G>
+__global__ void __launch_bounds__(256)
+    density_accum(const T* __restrict__ qf, const T* __restrict__ qb, DensityArgs d, double* __restrict__ raw,
+                  double* __restrict__ junc, double* __restrict__ qend) {
+    constexpr int LANES = 256 / G;
+    __shared__ double red[G > 1 ? G : 1][G > 1 ? LANES * P : 1];
+    const int64_t nr = d.nr, sl = (int64_t)d.M * nr;
+    const int lane = threadIdx.x % LANES, g = threadIdx.x / LANES;
+    const int64_t r = ((int64_t)blockIdx.x * LANES + lane) * P;
+    const bool in = r < nr;
+    double acc[3][P] = {};
+    // sum over the groups of v[], for the threads of group 0
+    auto over_groups = [&](double* v) {
+        if constexpr (G > 1) {
+            __syncthreads();
+#pragma unroll
+            for (int u = 0; u < P; ++u) red[g][lane * P + u] = v[u];
+            __syncthreads();
+            if (g == 0)
+#pragma unroll
+                for (int u = 0; u < P; ++u) {
+                    v[u] = red[0][lane * P + u];
+                    for (int q = 1; q < G; ++q) v[u] += red[q][lane * P + u];
                 }
-                acc *= d.ds / 3.0;
+        }
+    };
+    const int sj[3] = {d.nstart[1], d.nstart[2], d.nmax};
+    for (int s = 0; s <= d.nmax; ++s) {
+        Dots<T, P> dot;
+        if (in) {
+            const T* a = qf + s * sl + r;
+            const T* c = qb + s * sl + r;
+#pragma unroll 4
+            for (int i = g; i < d.M; i += G) {
+                T x[P], y[P];
+                if constexpr (P > 1) {
+                    vload<T>(a + i * nr, x);
+                    vload<T>(c + i * nr, y);
+                } else {
+                    x[0] = a[i * nr];
+                    y[0] = c[i * nr];
+                }
+#pragma unroll
+                for (int u = 0; u < P; ++u) dot.add(u, x[u], y[u]);
             }
-            raw[b * nr + r] = acc;
         }
-        const int sj[3] = {d.nstart[1], d.nstart[2], d.nmax};
-        for (int j = 0; j < 3; ++j) {
-            junc[j * nr + r] = dot_coeffs(qf + sj[j] * sl + r, qb + sj[j] * sl + r, d.M, nr);
+        double v[P];
+#pragma unroll
+        for (int u = 0; u < P; ++u) v[u] = dot.get(u);
+        for (int b = 0; b < 3; ++b) {
+            const int j = s - d.nstart[b], n = d.ns[b];
+            if (n <= 0 || j < 0 || j > n) continue;
+            const double wgt = (j == 0 || j == n) ? 1.0 : ((j & 1) ? 4.0 : 2.0);
+#pragma unroll
+            for (int u = 0; u < P; ++u) acc[b][u] += wgt * v[u];
         }
-        qend[r] = (double)qf[(int64_t)d.nmax * sl + r];
+        if (s == sj[0] || s == sj[1] || s == sj[2]) {
+            over_groups(v);
+            if (g == 0 && in)
+                for (int j = 0; j < 3; ++j)
+                    if (s == sj[j])
+#pragma unroll
+                        for (int u = 0; u < P; ++u) junc[j * nr + r + u] = v[u];
+        }
     }
-}
-
-// one J-list entry packed for a single broadcast load per entry (8 bytes
-// in FP32, 16 in FP64) instead of three loads from separate arrays
-template <typename T> struct alignas(sizeof(T) == 8 ? 16 : 8) JEnt {
-    T val;
-    int16_t row, col;
-};
-
-// shared-memory layout of the tiled density / tensor kernels:
-// sa[M][TILE] | sc[M][TILE] | jent[nj] | jptr[6]
-template <typename T> __host__ __device__ inline size_t slice_smem_bytes(int M, int nj, bool want_s) {
-    size_t b = 2 * sizeof(T) * (size_t)M * PointTile<T>::value;
-    if (want_s) b += sizeof(JEnt<T>) * (size_t)nj + sizeof(int) * 6;
-    return b;
-}
-
-template <typename T> struct SliceSmem {
-    T* sa;
-    T* sc;
-    JEnt<T>* jent;
-    int* jptr;
-};
-
-template <typename T> __device__ __forceinline__ SliceSmem<T> slice_smem(unsigned char* raw, int M, int nj) {
-    constexpr int TILE = PointTile<T>::value;
-    SliceSmem<T> m;
-    m.sa = reinterpret_cast<T*>(raw);
-    m.sc = m.sa + (size_t)M * TILE;
-    m.jent = reinterpret_cast<JEnt<T>*>(m.sc + (size_t)M * TILE);  // 2 M TILE sizeof(T) bytes in: 16-aligned
-    m.jptr = reinterpret_cast<int*>(m.jent + nj);
-    return m;
-}
-
-template <typename T> __device__ __forceinline__ void stage_jlists(const JLists& jl, const SliceSmem<T>& m) {
-    for (int e = threadIdx.x; e < jl.n; e += blockDim.x) {
-        JEnt<T> x;
-        x.val = (T)jl.val[e];
-        x.row = jl.row[e];
-        x.col = jl.col[e];
-        m.jent[e] = x;
+    for (int b = 0; b < 3; ++b) {
+        over_groups(acc[b]);
+        if (g == 0 && in)
+#pragma unroll
+            for (int u = 0; u < P; ++u) raw[b * nr + r + u] = acc[b][u] * (d.ds / 3.0);
     }
-    for (int e = threadIdx.x; e < 6; e += blockDim.x) m.jptr[e] = jl.ptr[e];
+    if (g == 0 && in)
+#pragma unroll
+        for (int u = 0; u < P; ++u) qend[r + u] = (double)qf[(int64_t)d.nmax * sl + r + u];
 }
 
-// stage the coefficient vectors of one slice for the tile's points (zeros
-// past the end of the grid), 16-byte vectors of consecutive points
+// shared-memory layout of the tiled density / tensor kernels: the tile of q*
+// [M][TILE], with the groups' partial sums over it [kGroups][W + 5][TILE]
+// afterwards | lists (with the tensor)
+template <typename T> __host__ __device__ inline size_t slice_tile_bytes(int M, bool want_s) {
+    const size_t red = sizeof(T) * (size_t)kGroups * (Dots<T, 1>::W + 5) * PointTile<T>::value;
+    const size_t tile = want_s ? sizeof(T) * (size_t)M * PointTile<T>::value : 0;
+    return red > tile ? red : tile;
+}
+template <typename T> __host__ __device__ inline size_t slice_smem_bytes(const ClassLists& jl, int M, bool want_s) {
+    return slice_tile_bytes<T>(M, want_s) + (want_s ? list_bytes<T>(jl.n, jl.ng, M) : 0);
+}
+
+// Sums of one slice at the tile's points: sum_i q_i q*_i (FP64 accuracy) and,
+// with the lists, the five forms q^T J_t q*.  Called by the whole CTA; the
+// partial sums over the groups of rows end in red.
 template <typename T>
-__device__ __forceinline__ void stage_tile(const T* __restrict__ a, const T* __restrict__ c, int M, int64_t nr,
-                                           int64_t r0, T* sa, T* sc) {
-    constexpr int TILE = PointTile<T>::value;
-    constexpr int V = 16 / sizeof(T);
-    for (int idx = threadIdx.x; idx < M * (TILE / V); idx += blockDim.x) {
-        const int i = idx / (TILE / V), k = (idx % (TILE / V)) * V;
-        const int64_t r = r0 + k;
-        T va[V] = {}, vc[V] = {};
-        if (r < nr) {
-            vload<T>(a + (int64_t)i * nr + r, va);
-            vload<T>(c + (int64_t)i * nr + r, vc);
+__device__ __forceinline__ void slice_sums(const T* __restrict__ a, const T* __restrict__ c, int M, int64_t nr, int64_t r0,
+                                           const ListSmem<T>* lists, T* tile) {
+    constexpr int TILE = PointTile<T>::value, P = Pts<T>::P, W = Dots<T, 1>::W;
+    const int k = (threadIdx.x % Pts<T>::LANES) * P, g = threadIdx.x / Pts<T>::LANES;
+    Dots<T, P> dot;
+    T f[5][P] = {};
+    if (lists) {
+        for (int idx = threadIdx.x; idx < M * (TILE / P); idx += blockDim.x) {
+            const int i = idx / (TILE / P), kk = (idx % (TILE / P)) * P;
+            T v[P];
+            vload<T>(c + (int64_t)i * nr + r0 + kk, v);
+            vstore<T>(tile + i * TILE + kk, v);
         }
-        vstore<T>(sa + i * TILE + k, va);
-        vstore<T>(sc + i * TILE + k, vc);
+        __syncthreads();
+        for (int row = g; row < M; row += kGroups) {
+            const int i = lists->order[row];
+            T q[P], p[P];
+            vload<T>(a + (int64_t)i * nr + r0 + k, q);
+            vload<T>(tile + i * TILE + k, p);
+#pragma unroll
+            for (int u = 0; u < P; ++u) dot.add(u, q[u], p[u]);
+            const uint16_t* pt = lists->ptr + 5 * i;
+            int e0 = pt[0];
+#pragma unroll
+            for (int t = 0; t < 5; ++t) {
+                const int e1 = pt[t + 1];
+                T y[P];
+                gather_sum<T>(*lists, e0, e1, tile + k, y);
+#pragma unroll
+                for (int u = 0; u < P; ++u) f[t][u] = fma(q[u], y[u], f[t][u]);
+                e0 = e1;
+            }
+        }
+        __syncthreads();  // the tile becomes the space of the partial sums
+    } else {
+#pragma unroll 4
+        for (int i = g; i < M; i += kGroups) {
+            T q[P], p[P];
+            vload<T>(a + (int64_t)i * nr + r0 + k, q);
+            vload<T>(c + (int64_t)i * nr + r0 + k, p);
+#pragma unroll
+            for (int u = 0; u < P; ++u) dot.add(u, q[u], p[u]);
+        }
     }
+    T* red = tile + (size_t)g * (W + 5) * TILE + k;
+#pragma unroll
+    for (int u = 0; u < P; ++u) {
+        dot.put(u, red + u, TILE);
+        if (lists)
+#pragma unroll
+            for (int t = 0; t < 5; ++t) red[(W + t) * TILE + u] = f[t][u];
+    }
+    __syncthreads();
 }
-
-// q^T J_t q* at one point from staged vectors (stride TILE) and staged lists
-template <typename T> __device__ __forceinline__ double jt_form(const SliceSmem<T>& m, int t, int k) {
-    constexpr int TILE = PointTile<T>::value;
-    T v = (T)0;
-    for (int e = m.jptr[t]; e < m.jptr[t + 1]; ++e) {
-        const JEnt<T> x = m.jent[e];
-        v += x.val * m.sa[x.row * TILE + k] * m.sc[x.col * TILE + k];
+// the tile's point k: the dot product, and tensor component t
+template <typename T> __device__ __forceinline__ double slice_dot(const T* red, int k) {
+    constexpr int TILE = PointTile<T>::value, W = Dots<T, 1>::W;
+    Dots<T, 1> dot;
+    for (int g = 0; g < kGroups; ++g) dot.merge(0, red + (size_t)g * (W + 5) * TILE + k, TILE);
+    return dot.get(0);
+}
+template <typename T> __device__ __forceinline__ double slice_form(const T* red, int t, int k) {
+    constexpr int TILE = PointTile<T>::value, W = Dots<T, 1>::W;
+    T x = (T)0, y = (T)0;  // component t; J11, J22: half sum and half difference
+    const int ta = t < 2 ? 0 : t;
+    for (int g = 0; g < kGroups; ++g) {
+        const T* w = red + ((size_t)g * (W + 5) + W) * TILE + k;
+        x += w[ta * TILE];
+        if (t < 2) y += w[TILE];
     }
-    return (double)v;
+    return (double)(t == 0 ? x + y : t == 1 ? x - y : x);
 }
 
 // orientation tensor per block (SCFT_Density_FE.f90:161-220):
-// sraw[b][t][r] = S1_s( q^T J_t q* ), t = 11, 22, 12, 13, 23; thread (k, t)
+// sraw[b][t][r] = S1_s( q^T J_t q* ), t = 11, 22, 12, 13, 23
 template <typename T>
-__global__ void __launch_bounds__(PointTile<T>::value * kSGroups)
-    stensor_accum(const T* __restrict__ qf, const T* __restrict__ qb, DensityArgs d, JLists jl,
+__global__ void __launch_bounds__(Pts<T>::THREADS)
+    stensor_accum(const T* __restrict__ qf, const T* __restrict__ qb, DensityArgs d, ClassLists jl,
                   double* __restrict__ sraw) {
-    constexpr int TILE = PointTile<T>::value;
+    constexpr int TILE = PointTile<T>::value, NT = Pts<T>::THREADS, Q = (5 * TILE + NT - 1) / NT;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const SliceSmem<T> m = slice_smem<T>(smem_raw, d.M, jl.n);
-    stage_jlists(jl, m);
-    const int64_t nr = d.nr;
-    const int64_t sl = (int64_t)d.M * nr;
-    const int k = threadIdx.x % TILE, t = threadIdx.x / TILE;
-    const int64_t r0 = (int64_t)blockIdx.x * TILE, r = r0 + k;
-    double acc[3] = {0.0, 0.0, 0.0};
-    for (int b = 0; b < 3; ++b) {
-        const int s0 = d.nstart[b], n = d.ns[b];
-        if (n <= 0) continue;
-        for (int s = s0; s <= s0 + n; ++s) {
-            const int j = s - s0;
-            const double wgt = (j == 0 || j == n) ? 1.0 : ((j & 1) ? 4.0 : 2.0);
-            __syncthreads();
-            stage_tile(qf + s * sl, qb + s * sl, d.M, nr, r0, m.sa, m.sc);
-            __syncthreads();
-            acc[b] += wgt * jt_form(m, t, k);
+    T* tile = reinterpret_cast<T*>(smem_raw);
+    const ListSmem<T> m = stage_lists<T>(jl, d.M, smem_raw + slice_tile_bytes<T>(d.M, true));
+    const int64_t nr = d.nr, sl = (int64_t)d.M * nr, r0 = (int64_t)blockIdx.x * TILE;
+    double acc[Q][3] = {};
+    for (int s = 0; s <= d.nmax; ++s) {
+        __syncthreads();  // lists staged / sums of the previous slice read
+        slice_sums<T>(qf + s * sl, qb + s * sl, d.M, nr, r0, &m, tile);
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            const int idx = threadIdx.x + q * NT;
+            if (idx >= 5 * TILE) break;
+            const double v = slice_form<T>(tile, idx / TILE, idx % TILE);
+#pragma unroll
+            for (int b = 0; b < 3; ++b) {
+                const int j = s - d.nstart[b], n = d.ns[b];
+                if (n <= 0 || j < 0 || j > n) continue;
+                acc[q][b] += ((j == 0 || j == n) ? 1.0 : ((j & 1) ? 4.0 : 2.0)) * v;
+            }
         }
     }
-    if (r < nr)
-        for (int b = 0; b < 3; ++b) sraw[((int64_t)b * 5 + t) * nr + r] = acc[b] * d.ds / 3.0;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        const int idx = threadIdx.x + q * NT;
+        if (idx >= 5 * TILE) break;
+#pragma unroll
+        for (int b = 0; b < 3; ++b)
+            sraw[((int64_t)b * 5 + idx / TILE) * nr + r0 + idx % TILE] = acc[q][b] * d.ds / 3.0;
+    }
 }
 
 // Streamed form of density_accum / stensor_accum: one slice s per launch,
 // issued by the backward sweep right after q*(s) is computed (descending s),
 // so the q* slices need not be stored.  Same Simpson weights per block.  One
-// CTA per tile of points; the tile's coefficient vectors of q(s) and q*(s)
-// are staged in shared memory once.
-// One CTA walks tiles of TILE points of one instance; thread (k, g): point k,
-// group g (g = 0 the densities, g = t the tensor component t when want_s;
-// blockDim = TILE * kSGroups when any instance of the launch wants S).
+// CTA walks tiles of TILE points of one instance.
+// 128^3, L = 12 with the tensor in FP32: 9.9 -> 2.4 ms a launch.
 template <typename T>
 __device__ __forceinline__ void density_slice_tiles(const T* __restrict__ a, const T* __restrict__ c,
-                                                    const DensityArgs& d, int s, int want_s, const JLists& jl,
+                                                    const DensityArgs& d, int s, int want_s, const ClassLists& jl,
                                                     double* __restrict__ raw, double* __restrict__ junc,
                                                     double* __restrict__ qend, double* __restrict__ sraw) {
     constexpr int TILE = PointTile<T>::value;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const SliceSmem<T> m = slice_smem<T>(smem_raw, d.M, want_s ? jl.n : 0);
-    if (want_s) stage_jlists(jl, m);
+    T* tile = reinterpret_cast<T*>(smem_raw);
+    ListSmem<T> m{};
+    if (want_s) m = stage_lists<T>(jl, d.M, smem_raw + slice_tile_bytes<T>(d.M, true));
     const int64_t nr = d.nr;
     double wgt[3];
-    bool any = false;
     for (int b = 0; b < 3; ++b) {
         const int j = s - d.nstart[b], n = d.ns[b];
-        wgt[b] = 0.0;
-        if (n > 0 && j >= 0 && j <= n) {
-            wgt[b] = (j == 0 || j == n) ? 1.0 : ((j & 1) ? 4.0 : 2.0);
-            any = true;
-        }
+        wgt[b] = (n > 0 && j >= 0 && j <= n) ? ((j == 0 || j == n) ? 1.0 : ((j & 1) ? 4.0 : 2.0)) : 0.0;
     }
     const int sj[3] = {d.nstart[1], d.nstart[2], d.nmax};
     const double scl = d.ds / 3.0;
-    const int k = threadIdx.x % TILE, g = threadIdx.x / TILE;
     for (int64_t r0 = (int64_t)blockIdx.x * TILE; r0 < nr; r0 += (int64_t)gridDim.x * TILE) {
-        __syncthreads();  // lists staged / previous tile consumed
-        stage_tile(a, c, d.M, nr, r0, m.sa, m.sc);
-        __syncthreads();
-        const int64_t r = r0 + k;
-        if (r >= nr) continue;
-        if (g == 0) {
-            const double sum = dot_coeffs(m.sa + k, m.sc + k, d.M, (int64_t)TILE);
-            if (any)
+        __syncthreads();  // lists staged / previous tile's sums read
+        slice_sums<T>(a, c, d.M, nr, r0, want_s ? &m : nullptr, tile);
+        for (int idx = threadIdx.x; idx < (want_s ? 6 : 1) * TILE; idx += blockDim.x) {
+            const int t = idx / TILE - 1, k = idx % TILE;
+            const int64_t r = r0 + k;
+            if (t < 0) {
+                const double sum = slice_dot<T>(tile, k);
                 for (int b = 0; b < 3; ++b)
                     if (wgt[b] != 0.0) raw[b * nr + r] += wgt[b] * sum;
-            for (int j = 0; j < 3; ++j)
-                if (s == sj[j]) junc[j * nr + r] = sum;
-            if (s == d.nmax) qend[r] = (double)a[r];
-            if (s == 0)  // last slice of the backward sweep
-                for (int b = 0; b < 3; ++b) raw[b * nr + r] *= scl;
-        }
-        if (want_s && g < 5) {
-            if (any) {
-                const double st = jt_form(m, g, k);
-                for (int b = 0; b < 3; ++b)
-                    if (wgt[b] != 0.0) sraw[((int64_t)b * 5 + g) * nr + r] += wgt[b] * st;
+                for (int j = 0; j < 3; ++j)
+                    if (s == sj[j]) junc[j * nr + r] = sum;
+                if (s == d.nmax) qend[r] = (double)a[r];
+                if (s == 0)  // last slice of the backward sweep
+                    for (int b = 0; b < 3; ++b) raw[b * nr + r] *= scl;
+            } else {
+                const double st = slice_form<T>(tile, t, k);
+                for (int b = 0; b < 3; ++b) {
+                    double* o = sraw + ((int64_t)b * 5 + t) * nr + r;
+                    if (wgt[b] != 0.0) *o += wgt[b] * st;
+                    if (s == 0) *o *= scl;
+                }
             }
-            if (s == 0)
-                for (int b = 0; b < 3; ++b) sraw[((int64_t)b * 5 + g) * nr + r] *= scl;
         }
     }
 }
 
 template <typename T>
-__global__ void __launch_bounds__(PointTile<T>::value * kSGroups)
-    density_slice(const T* __restrict__ a, const T* __restrict__ c, DensityArgs d, int s, int want_s, JLists jl,
+__global__ void __launch_bounds__(Pts<T>::THREADS)
+    density_slice(const T* __restrict__ a, const T* __restrict__ c, DensityArgs d, int s, int want_s, ClassLists jl,
                   double* __restrict__ raw, double* __restrict__ junc, double* __restrict__ qend,
                   double* __restrict__ sraw) {
     density_slice_tiles<T>(a, c, d, s, want_s, jl, raw, junc, qend, sraw);
 }
 
 template <typename T>
-__global__ void __launch_bounds__(PointTile<T>::value * kSGroups)
+__global__ void __launch_bounds__(Pts<T>::THREADS)
     density_slice_batched(const SliceBatchArgs<T>* __restrict__ args, int s) {
     const SliceBatchArgs<T> g = args[blockIdx.y];
     density_slice_tiles<T>(g.qf + (int64_t)s * g.sl, g.qb + (int64_t)(s & 3) * g.sl, g.d, s, g.want_s, g.jl, g.raw,
@@ -524,39 +705,43 @@ static unsigned tile_grid(int64_t nr, int tile) {
 }
 
 template <typename T>
-void launch_ms_term(const T* h1, const T* h2, const T* h3, int order, const double* mop, const ThetaLists& tl,
+void launch_ms_term(const T* h1, const T* h2, const T* h3, int order, const double* mop, const ClassLists& tl,
                     double ds, double thresh, int M, int64_t nr, T* out, cudaStream_t st) {
-    constexpr int TILE = PointTile<T>::value;
-    ms_term<T><<<tile_grid(nr, TILE), TILE * kMsGroups, ms_smem_bytes<T>(tl.n, M), st>>>(h1, h2, h3, order, mop, tl,
-                                                                                      ds, thresh, M, nr, out);
+    ms_term<T><<<tile_grid(nr, PointTile<T>::value), Pts<T>::THREADS, ms_smem_bytes<T>(tl, M), st>>>(
+        h1, h2, h3, order, mop, tl, ds, thresh, M, nr, out);
 }
 template <typename T>
 void launch_density(const T* qf, const T* qb, const DensityArgs& d, double* raw, double* junc, double* qend,
                     cudaStream_t st) {
-    density_accum<T><<<grid_for(d.nr), 256, 0, st>>>(qf, qb, d, raw, junc, qend);
+    constexpr int P = Pts<T>::P;
+    const int64_t nr = d.nr;
+    // P points a thread once that makes 3 CTAs for every SM, with the coefficients
+    // in two groups if need be; one point and eight groups on small grids
+    if (nr / (256 * P) >= 456)
+        density_accum<T, P, 1><<<(unsigned)((nr / P + 255) / 256), 256, 0, st>>>(qf, qb, d, raw, junc, qend);
+    else if (nr / (128 * P) >= 456)
+        density_accum<T, P, 2><<<(unsigned)((nr / P + 127) / 128), 256, 0, st>>>(qf, qb, d, raw, junc, qend);
+    else
+        density_accum<T, 1, 8><<<(unsigned)((nr + 31) / 32), 256, 0, st>>>(qf, qb, d, raw, junc, qend);
 }
 template <typename T>
-void launch_stensor(const T* qf, const T* qb, const DensityArgs& d, const JLists& jl, double* sraw, cudaStream_t st) {
-    constexpr int TILE = PointTile<T>::value;
-    stensor_accum<T><<<(unsigned)((d.nr + TILE - 1) / TILE), TILE * kSGroups, slice_smem_bytes<T>(d.M, jl.n, true),
-                       st>>>(qf, qb, d, jl, sraw);
+void launch_stensor(const T* qf, const T* qb, const DensityArgs& d, const ClassLists& jl, double* sraw, cudaStream_t st) {
+    stensor_accum<T><<<(unsigned)(d.nr / PointTile<T>::value), Pts<T>::THREADS, slice_smem_bytes<T>(jl, d.M, true), st>>>(
+        qf, qb, d, jl, sraw);
 }
 
 template <typename T>
-void launch_density_slice(const T* qf_s, const T* qb_s, const DensityArgs& d, int s, int want_s, const JLists& jl,
+void launch_density_slice(const T* qf_s, const T* qb_s, const DensityArgs& d, int s, int want_s, const ClassLists& jl,
                           double* raw, double* junc, double* qend, double* sraw, cudaStream_t st) {
-    constexpr int TILE = PointTile<T>::value;
-    density_slice<T><<<tile_grid(d.nr, TILE), TILE * (want_s ? kSGroups : 1),
-                       slice_smem_bytes<T>(d.M, jl.n, want_s != 0), st>>>(qf_s, qb_s, d, s, want_s, jl, raw, junc,
-                                                                          qend, sraw);
+    density_slice<T><<<tile_grid(d.nr, PointTile<T>::value), Pts<T>::THREADS, slice_smem_bytes<T>(jl, d.M, want_s != 0),
+                       st>>>(qf_s, qb_s, d, s, want_s, jl, raw, junc, qend, sraw);
 }
 
 template <typename T>
-void launch_density_slice_batched(const SliceBatchArgs<T>* args, int count, int64_t max_nr, int s, int M, int nj,
-                                  int any_s, cudaStream_t st) {
-    constexpr int TILE = PointTile<T>::value;
-    density_slice_batched<T><<<dim3(tile_grid(max_nr, TILE), count), TILE * (any_s ? kSGroups : 1),
-                               slice_smem_bytes<T>(M, nj, any_s != 0), st>>>(args, s);
+void launch_density_slice_batched(const SliceBatchArgs<T>* args, int count, int64_t max_nr, int s, int M,
+                                  const ClassLists& jl, int any_s, cudaStream_t st) {
+    density_slice_batched<T><<<dim3(tile_grid(max_nr, PointTile<T>::value), count), Pts<T>::THREADS,
+                               slice_smem_bytes<T>(jl, M, any_s != 0), st>>>(args, s);
 }
 
 void launch_s3(const double* a, int nsum, int64_t stride, const S3Args& s, double* part, double* out,
@@ -582,15 +767,15 @@ void launch_nonfinite(const double* a, int64_t n, int* flag, cudaStream_t st) {
     template void launch_to_reference<T>(const T*, double*, int, int64_t, cudaStream_t);                          \
     template void launch_set_delta<T>(T*, int, int64_t, cudaStream_t);                                           \
     template void launch_make_cf<T>(const double*, T*, double, double, int64_t, cudaStream_t);                    \
-    template void launch_ms_term<T>(const T*, const T*, const T*, int, const double*, const ThetaLists&, double,  \
+    template void launch_ms_term<T>(const T*, const T*, const T*, int, const double*, const ClassLists&, double,  \
                                     double, int, int64_t, T*, cudaStream_t);                                     \
     template void launch_density<T>(const T*, const T*, const DensityArgs&, double*, double*, double*,           \
                                     cudaStream_t);                                                               \
-    template void launch_stensor<T>(const T*, const T*, const DensityArgs&, const JLists&, double*, cudaStream_t); \
-    template void launch_density_slice<T>(const T*, const T*, const DensityArgs&, int, int, const JLists&, double*, \
+    template void launch_stensor<T>(const T*, const T*, const DensityArgs&, const ClassLists&, double*, cudaStream_t); \
+    template void launch_density_slice<T>(const T*, const T*, const DensityArgs&, int, int, const ClassLists&, double*, \
                                           double*, double*, double*, cudaStream_t);                              \
-    template void launch_density_slice_batched<T>(const SliceBatchArgs<T>*, int, int64_t, int, int, int, int,        \
-                                                  cudaStream_t);
+    template void launch_density_slice_batched<T>(const SliceBatchArgs<T>*, int, int64_t, int, int,                  \
+                                                  const ClassLists&, int, cudaStream_t);
 WLC_INST(double)
 WLC_INST(float)
 #undef WLC_INST

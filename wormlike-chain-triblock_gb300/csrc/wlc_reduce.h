@@ -28,23 +28,23 @@ struct FeArgs {
     int ms;
 };
 
-// union of the five Theta basis tensors: entry e couples (row, col) with
-// values val[5e + c], c = T1122, T33, T12, T13, T23
-struct ThetaLists {
-    int n;
-    const int* rowptr;  // [M+1]: entries of row i at [rowptr[i], rowptr[i+1]) (entries are sorted by row)
-    const int16_t* row;
+// Sparse coupling tensors of five components, row by row and component by
+// component: entries of (row i, component c) at [ptr[5i+c], ptr[5i+c+1]).
+// Theta: components T1122, T33, T12, T13, T23; pairs (i, j) with several
+// nonzero components are kept apart (g*, all five values), because the
+// threshold applies to their sum.  J: components (J11+J22)/2, (J11-J22)/2,
+// J12, J13, J23 (for one pair (i, j) most components vanish: m of the two
+// harmonics picks one).
+struct ClassLists {
+    int n, ng;
+    const uint16_t* ptr;    // [5M + 1]
     const int16_t* col;
     const double* val;
-};
-
-// five J lists (J11, J22, J12, J13, J23) concatenated; ptr[6]
-struct JLists {
-    int n;  // total entries (ptr[5])
-    const int* ptr;
-    const int16_t* row;
-    const int16_t* col;
-    const double* val;
+    double vmin[5], vmax[5];  // |val| over each component
+    const uint16_t* gptr;   // [M + 1]
+    const int16_t* gcol;
+    const double* gval;     // [ng][5]
+    const int16_t* order;   // rows, longest first
 };
 
 // points per CTA of the tiled per-point coefficient kernels (ms_term,
@@ -57,8 +57,6 @@ template <typename T> struct PointTile {
 // current device; call on each device before any stream capture (repeat
 // calls on a device return at once)
 cudaError_t prepare_reduce_kernels();
-constexpr int kMsGroups = 4;  // ms_term: row groups per point (threads per point)
-constexpr int kSGroups = 5;   // orientation tensor: one thread per component per point
 
 template <typename T> void launch_to_internal(const double* ref, T* out, int M, int64_t nr, cudaStream_t st);
 template <typename T> void launch_to_reference(const T* in, double* ref, int M, int64_t nr, cudaStream_t st);
@@ -66,13 +64,13 @@ template <typename T> void launch_set_delta(T* q, int M, int64_t nr, cudaStream_
 template <typename T>
 void launch_make_cf(const double* w, T* cf, double ds, double third, int64_t nr, cudaStream_t st);
 template <typename T>
-void launch_ms_term(const T* h1, const T* h2, const T* h3, int order, const double* mop, const ThetaLists& tl,
+void launch_ms_term(const T* h1, const T* h2, const T* h3, int order, const double* mop, const ClassLists& tl,
                     double ds, double thresh, int M, int64_t nr, T* out, cudaStream_t st);
 template <typename T>
 void launch_density(const T* qf, const T* qb, const DensityArgs& d, double* raw, double* junc, double* qend,
                     cudaStream_t st);
 template <typename T>
-void launch_stensor(const T* qf, const T* qb, const DensityArgs& d, const JLists& jl, double* sraw, cudaStream_t st);
+void launch_stensor(const T* qf, const T* qb, const DensityArgs& d, const ClassLists& jl, double* sraw, cudaStream_t st);
 // one contour slice s of the streamed density integrals (q(s), q*(s) given):
 // raw/sraw += Simpson weight x q.q* for the blocks containing s, junction
 // and Q(end) slices copied; at the last slice (s = 0) scaled by ds/3
@@ -84,18 +82,18 @@ template <typename T> struct SliceBatchArgs {
     int64_t sl;
     DensityArgs d;
     int want_s;
-    JLists jl;
+    ClassLists jl;
     double* raw;
     double* junc;
     double* qend;
     double* sraw;
 };
 template <typename T>
-void launch_density_slice_batched(const SliceBatchArgs<T>* args, int count, int64_t max_nr, int s, int M, int nj,
-                                  int any_s, cudaStream_t st);
+void launch_density_slice_batched(const SliceBatchArgs<T>* args, int count, int64_t max_nr, int s, int M,
+                                  const ClassLists& jl, int any_s, cudaStream_t st);
 
 template <typename T>
-void launch_density_slice(const T* qf_s, const T* qb_s, const DensityArgs& d, int s, int want_s, const JLists& jl,
+void launch_density_slice(const T* qf_s, const T* qb_s, const DensityArgs& d, int s, int want_s, const ClassLists& jl,
                           double* raw, double* junc, double* qend, double* sraw, cudaStream_t st);
 void launch_s3(const double* a, int nsum, int64_t stride, const S3Args& s, double* part, double* out,
                cudaStream_t st);
