@@ -174,12 +174,15 @@ template <> struct Dft<6> : DftCT<2, 3> {};
 template <> struct Dft<16> : DftCT<4, 4> {};
 
 // ------------------------------------------------------------ line plans
+// (16 as 4 x 4: one 16-point transform a thread left most of a small grid's
+// threads idle and each fetched its straight-line code cold; FP64 16^3, L = 2:
+// pass A 12.8 -> 9.1, B 39 -> 29, C 12.5 -> 8.5 us, FP32 within 3 % either way)
 template <int N> struct Plan;
 template <> struct Plan<4> { static constexpr int N1 = 4, N2 = 1; };
 template <> struct Plan<6> { static constexpr int N1 = 6, N2 = 1; };
 template <> struct Plan<8> { static constexpr int N1 = 8, N2 = 1; };
 template <> struct Plan<12> { static constexpr int N1 = 4, N2 = 3; };
-template <> struct Plan<16> { static constexpr int N1 = 16, N2 = 1; };
+template <> struct Plan<16> { static constexpr int N1 = 4, N2 = 4; };
 template <> struct Plan<24> { static constexpr int N1 = 8, N2 = 3; };
 template <> struct Plan<32> { static constexpr int N1 = 8, N2 = 4; };
 template <> struct Plan<40> { static constexpr int N1 = 8, N2 = 5; };
