@@ -139,44 +139,78 @@ __global__ void __launch_bounds__(128) gather_gemm(const bf16* __restrict__ A, i
     }
 }
 
-// Weight gradient, one kk per CTA column (blockIdx.z = kk * splits + split):
+// Weight gradient, one (kk, split) per warp (z = kk * splits + split):
 // part[split][kk][ci][co] = sum over q in the split's range of
-// x[nb_fwd(q,kk)][ci] dz[q][co].  A warp computes 16 ci x 16 co.
-__global__ void __launch_bounds__(32) wgrad(const bf16* __restrict__ X, int Ci, const bf16* __restrict__ dZ, int Co,
-                                            int Mq, int gi, int go, int stride, int splits,
-                                            float* __restrict__ part) {
-    const int lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
-    const int ci0 = blockIdx.x * 16, co0 = blockIdx.y * 16;
-    const int kk = blockIdx.z / splits, sp = blockIdx.z % splits;
+// x[nb_fwd(q,kk)][ci] dz[q][co].  A warp computes 16 ci x 16 NB co, 16 points
+// q at a time: rows of x and dz come in 16-byte pieces (the next ones in
+// flight while these are multiplied) and are transposed by ldmatrix on the
+// way to the tensor core.  Element-wise 2-byte gathers bound the earlier form:
+// the largest layer at 32^3, width 32 844 -> 92 us.
+template <int NB>
+__global__ void __launch_bounds__(128) wgrad(const bf16* __restrict__ X, int Ci, const bf16* __restrict__ dZ, int Co,
+                                             int Mq, int gi, int go, int stride, int splits,
+                                             float* __restrict__ part) {
+    // row strides of 48 and 32 NB + 16 bytes put the 8 rows of an ldmatrix on distinct banks
+    constexpr int XS = 24, ZS = 16 * NB + 8;
+    __shared__ __align__(16) bf16 sx[4][2][16 * XS], sz[4][2][16 * ZS];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
+    const int zi = blockIdx.z * 4 + warp;
+    if (zi >= 27 * splits) return;
+    const int ci0 = blockIdx.x * 16, co0 = blockIdx.y * 16 * NB;
+    const int kk = zi / splits, sp = zi % splits;
     const int per = ((Mq + splits - 1) / splits + 15) / 16 * 16;
     const int qb = sp * per, qe = min(Mq, qb + per);
-    float c[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
-    auto xval = [&](int q, int ci) -> bf16 {
-        return q < qe ? X[(size_t)nb_fwd(q, kk, gi, go, stride) * Ci + ci] : __float2bfloat16(0.0f);
-    };
-    auto zval = [&](int q, int co) -> bf16 { return q < qe ? dZ[(size_t)q * Co + co] : __float2bfloat16(0.0f); };
-    for (int q0 = qb; q0 < qe; q0 += 16) {
-        const int qa = q0 + tig * 2;
-        const uint32_t a0 = pack2(xval(qa, ci0 + gid), xval(qa + 1, ci0 + gid));
-        const uint32_t a1 = pack2(xval(qa, ci0 + gid + 8), xval(qa + 1, ci0 + gid + 8));
-        const uint32_t a2 = pack2(xval(qa + 8, ci0 + gid), xval(qa + 9, ci0 + gid));
-        const uint32_t a3 = pack2(xval(qa + 8, ci0 + gid + 8), xval(qa + 9, ci0 + gid + 8));
+    const int row = lane >> 1, half = (lane & 1) * 8;
+    uint4 rx, rz[NB];
+    auto fetch = [&](int q) {
+        rx = make_uint4(0, 0, 0, 0);
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const int co = co0 + j * 8 + gid;
-            mma_bf16(c[j], a0, a1, a2, a3, pack2(zval(qa, co), zval(qa + 1, co)),
-                     pack2(zval(qa + 8, co), zval(qa + 9, co)));
+        for (int j = 0; j < NB; ++j) rz[j] = rx;
+        if (q < qe) {
+            rx = *reinterpret_cast<const uint4*>(X + (size_t)nb_fwd(q, kk, gi, go, stride) * Ci + ci0 + half);
+#pragma unroll
+            for (int j = 0; j < NB; ++j)
+                rz[j] = *reinterpret_cast<const uint4*>(dZ + (size_t)q * Co + co0 + 16 * j + half);
+        }
+    };
+    auto ldsm4t = [](uint32_t r[4], const bf16* p) {
+        const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                     : "r"(a)
+                     : "memory");
+    };
+    float c[NB][2][4] = {};
+    fetch(qb + row);
+    int buf = 0;
+    for (int q0 = qb; q0 < qe; q0 += 16, buf ^= 1) {
+        *reinterpret_cast<uint4*>(&sx[warp][buf][row * XS + half]) = rx;
+#pragma unroll
+        for (int j = 0; j < NB; ++j) *reinterpret_cast<uint4*>(&sz[warp][buf][row * ZS + 16 * j + half]) = rz[j];
+        __syncwarp();
+        fetch(q0 + 16 + row);
+        // 8 x 8 pieces (q, ci): (0, 0), (0, 8), (8, 0), (8, 8)
+        uint32_t a[4];
+        ldsm4t(a, &sx[warp][buf][((lane & 7) + (lane >> 4) * 8) * XS + ((lane >> 3) & 1) * 8]);
+#pragma unroll
+        for (int j = 0; j < NB; ++j) {
+            uint32_t b[4];  // pieces (q, co): (0, 0), (8, 0), (0, 8), (8, 8)
+            ldsm4t(b, &sz[warp][buf][((lane & 7) + ((lane >> 3) & 1) * 8) * ZS + 16 * j + (lane >> 4) * 8]);
+            mma_bf16(c[j][0], a[0], a[1], a[2], a[3], b[0], b[1]);
+            mma_bf16(c[j][1], a[0], a[1], a[2], a[3], b[2], b[3]);
         }
     }
     float* out = part + ((size_t)sp * 27 + kk) * Ci * Co;
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-        const int col = co0 + j * 8 + tig * 2;
-        out[(size_t)(ci0 + gid) * Co + col] = c[j][0];
-        out[(size_t)(ci0 + gid) * Co + col + 1] = c[j][1];
-        out[(size_t)(ci0 + gid + 8) * Co + col] = c[j][2];
-        out[(size_t)(ci0 + gid + 8) * Co + col + 1] = c[j][3];
-    }
+    for (int j = 0; j < NB; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int col = co0 + 16 * j + 8 * h + tig * 2;
+            out[(size_t)(ci0 + gid) * Co + col] = c[j][h][0];
+            out[(size_t)(ci0 + gid) * Co + col + 1] = c[j][h][1];
+            out[(size_t)(ci0 + gid + 8) * Co + col] = c[j][h][2];
+            out[(size_t)(ci0 + gid + 8) * Co + col + 1] = c[j][h][3];
+        }
 }
 
 // grad[e] += sum over splits of part[split][e] (fixed order)
@@ -188,13 +222,24 @@ __global__ void sum_splits(const float* __restrict__ part, int splits, int64_t n
     }
 }
 
-// db[co] += sum_q dz[q][co]
-__global__ void bias_grad(const bf16* __restrict__ dZ, int Co, int Mq, float* __restrict__ db) {
-    const int co = blockIdx.x * blockDim.x + threadIdx.x;
-    if (co >= Co) return;
+// part[chunk][co] = sum of dz[q][co] over the chunk's rows q (16 channels a
+// CTA, 16 rows at a time; sum_splits adds the chunks).  One thread a channel
+// over all rows took 0.9 ms for each layer at 32^3, most of a training sample.
+__global__ void __launch_bounds__(256) bias_partial(const bf16* __restrict__ dZ, int Co, int Mq,
+                                                    float* __restrict__ part) {
+    __shared__ float sm[16][17];
+    const int c = threadIdx.x & 15, r = threadIdx.x >> 4, co = blockIdx.x * 16 + c;
+    const int per = (Mq + gridDim.y - 1) / gridDim.y;
+    const int qb = blockIdx.y * per, qe = min(Mq, qb + per);
     float s = 0.0f;
-    for (int q = 0; q < Mq; ++q) s += __bfloat162float(dZ[(size_t)q * Co + co]);
-    db[co] += s;
+#pragma unroll 4
+    for (int q = qb + r; q < qe; q += 16) s += __bfloat162float(dZ[(size_t)q * Co + co]);
+    sm[r][c] = s;
+    __syncthreads();
+    if (r == 0) {
+        for (int k = 1; k < 16; ++k) s += sm[k][c];
+        part[(size_t)blockIdx.y * Co + co] = s;
+    }
 }
 
 // dz = bf16(dy * relu'(y)) (relu = 0: no mask)
@@ -475,11 +520,18 @@ static void conv_bwd(wlc_net* n, const Layer& l, const bf16* x, const bf16* y, c
     const int64_t Mq = pts(l.gout), Mp = pts(l.gin);
     relu_back<<<gridn(Mq * l.co), 256, 0, n->st>>>(dy, y, l.relu, Mq * l.co, n->dz);
     const int splits = (int)std::max<int64_t>(1, std::min<int64_t>(n->splits, Mq / 16));
-    wgrad<<<dim3(l.ci / 16, l.co / 16, 27 * splits), 32, 0, n->st>>>(x, l.ci, n->dz, l.co, (int)Mq, l.gin, l.gout,
-                                                                     l.stride, splits, n->part);
+    const unsigned gz = (unsigned)((27 * splits + 3) / 4);
+    if (l.co % 32 == 0)
+        wgrad<2><<<dim3(l.ci / 16, l.co / 32, gz), 128, 0, n->st>>>(x, l.ci, n->dz, l.co, (int)Mq, l.gin, l.gout,
+                                                                   l.stride, splits, n->part);
+    else
+        wgrad<1><<<dim3(l.ci / 16, l.co / 16, gz), 128, 0, n->st>>>(x, l.ci, n->dz, l.co, (int)Mq, l.gin, l.gout,
+                                                                   l.stride, splits, n->part);
     const int64_t nw = (int64_t)27 * l.ci * l.co;
     sum_splits<<<gridn(nw), 256, 0, n->st>>>(n->part, splits, nw, n->g + l.woff);
-    bias_grad<<<(l.co + 63) / 64, 64, 0, n->st>>>(n->dz, l.co, (int)Mq, n->g + l.boff);
+    const int chunks = (int)std::max<int64_t>(1, std::min<int64_t>(64, Mq / 256));  // fits part: 64 co < 27 ci co
+    bias_partial<<<dim3(l.co / 16, chunks), 256, 0, n->st>>>(n->dz, l.co, (int)Mq, n->part);
+    sum_splits<<<gridn(l.co), 256, 0, n->st>>>(n->part, chunks, l.co, n->g + l.boff);
     if (dx) {
         const dim3 grid((unsigned)((Mp + 63) / 64), l.ci / 16);
         gather_gemm<1><<<grid, 128, 0, n->st>>>(n->dz, l.co, l.wb, l.ci, (int)Mp, l.gin, l.gout, l.stride, nullptr, 0,
