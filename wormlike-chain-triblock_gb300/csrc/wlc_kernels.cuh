@@ -16,7 +16,7 @@
 namespace wlc {
 
 // Element stride of one packed x row in the shared buffers of passes A and
-// C: N + 1 (odd), so that the line-fastest x-FFT work split puts the lanes
+// C of the FP64 form: N + 1 (odd), so that the line-fastest x-FFT work split puts the lanes
 // of a warp on distinct banks.  (N/2) rows of a plane then take
 // (N/2)(N+1) elements, an even count for the supported N (multiples of 4),
 // which keeps the buffers after them 16-byte aligned.

@@ -89,38 +89,16 @@ __device__ __forceinline__ void cp_async16(void* sdst, const void* gsrc) {
     const unsigned sa = (unsigned)__cvta_generic_to_shared(sdst);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gsrc) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int n> __device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(n) : "memory");
-}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // The half-spectrum planes of a CTA are kept z-fastest, out[(ky*NKX + kx)*Z + zz],
 // so that the Z values of one (col, i) run in phat move as one 32-byte chunk.
 
+// ------------------------------------------------ FP64 form: passes A and C
 // x-FFTs of ZB planes of packed row pairs (zb: ZB consecutive (N/2) x N
-// blocks, row stride xrow(N)), split into two half spectra each: planes zz0 .. zz0+ZB-1 of out
-// (the y-FFTs of all planes follow in one batched call, y_planes)
-template <typename T, int N, int Z, int ZB>
-__device__ __forceinline__ void fwd_x_planes(typename cvec<T>::t* zb, typename cvec<T>::t* out, int zz0,
-                                             const typename cvec<T>::t* tw) {
-    using C = typename cvec<T>::t;
-    constexpr int NKX = N / 2 + 1;
-    constexpr int XR = xrow(N);
-    fft_nat2perm<N, -1>(zb, ZB * (N / 2), 1, XR, tw);
-    for (int t = threadIdx.x; t < ZB * (N / 2) * NKX; t += blockDim.x) {
-        const int q = t / ((N / 2) * NKX), e = t % ((N / 2) * NKX);
-        const int p = e / NKX, k = e % NKX;
-        const C* zq = zb + (size_t)q * xplane(N);
-        const C zk = zq[p * XR + perm_pos<N>(k)];
-        const C zm = zq[p * XR + perm_pos<N>((N - k) % N)];
-        out[((2 * p) * NKX + k) * Z + zz0 + q] = cmk<C>((T)0.5 * (zk.x + zm.x), (T)0.5 * (zk.y - zm.y));
-        out[((2 * p + 1) * NKX + k) * Z + zz0 + q] = cmk<C>((T)0.5 * (zk.y + zm.y), (T)0.5 * (zm.x - zk.x));
-    }
-    __syncthreads();
-}
-
-// the same in the FP64 form: fixed-point half spectra (twice their value)
-// with one exponent per row pair in el
+// blocks, row stride xrow(N)), split into two half spectra each: planes zz0 ..
+// zz0+ZB-1 of out (the y-FFTs of all planes follow in one batched call), as
+// fixed-point numbers (twice their value) with one exponent per row pair in el
 template <int N, int Z, int ZB>
 __device__ __forceinline__ void fwd_x_planes_fx(double2* zb, fxc* out, int zz0, const fxw* tw, int16_t* es, int16_t* el) {
     constexpr int NKX = N / 2 + 1;
@@ -136,14 +114,6 @@ __device__ __forceinline__ void fwd_x_planes_fx(double2* zb, fxc* out, int zz0, 
         out[((2 * p + 1) * NKX + k) * Z + zz0 + q] = fxc{zk.y + zm.y, zm.x - zk.x};
     }
     __syncthreads();
-}
-
-// y-FFTs of every (kx, plane) line of out: line kx*Z + zz starts at out + kx*Z + zz,
-// element ky at stride NKX*Z
-template <typename T, int N, int Z, int DIR>
-__device__ __forceinline__ void y_planes(typename cvec<T>::t* out, const typename cvec<T>::t* tw) {
-    constexpr int NKX = N / 2 + 1;
-    fft_nat2perm<N, DIR>(out, NKX * Z, NKX * Z, 1, tw);
 }
 
 // one Z-run per (ky, kx) from the half spectra to phat, in 16-byte pieces
@@ -176,86 +146,70 @@ template <typename T, int N, int V> struct XyShape {
     static constexpr int ZB = (V & 2) ? Z : 1;
 };
 
-template <typename T, int N, bool B = false, int V = 0>
-__global__ void __launch_bounds__(512) rhs_fft_xy(StepArgs<T> a0, const StepArgs<T>* __restrict__ batch) {
-    const StepArgs<T> a = pick_args<B>(a0, batch);
-    using C = typename cvec<T>::t;
+template <int N, int V = 0>
+__global__ void __launch_bounds__(512) rhs_fft_xy(StepArgs<double> a) {
+    using T = double;
+    using C = double2;
     constexpr int Z = XyShape<T, N, V>::Z, ZB = XyShape<T, N, V>::ZB;
     constexpr int NKX = N / 2 + 1;
     constexpr int NR = N * N * N;
     constexpr int PB = (N / 2) * N;  // packed row pairs per plane
     constexpr int XR = xrow(N), PBS = xplane(N);
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    C* tw = reinterpret_cast<C*>(smem_raw);
-    C* zb = tw + N;                  // ZB x (N/2) x N packed row pairs (row stride XR)
-    C* out = zb + (size_t)ZB * PBS;  // N x NKX x Z half spectra
+    fxw* twx = reinterpret_cast<fxw*>(smem_raw);
+    C* zb = reinterpret_cast<C*>(twx + N);  // ZB x (N/2) x N packed row pairs (row stride XR)
+    C* out = zb + (size_t)ZB * PBS;         // N x NKX x Z half spectra
+    int16_t* el = reinterpret_cast<int16_t*>(out + (size_t)Z * N * NKX);  // exponents per line, then scratch
+    int16_t* es = el + Z * NKX;
     const int i = blockIdx.y;
     const int z0 = blockIdx.x * Z;
-    fxw* twx = reinterpret_cast<fxw*>(smem_raw);
-    int16_t* el = reinterpret_cast<int16_t*>(out + (size_t)Z * N * NKX);  // FP64 form: exponents per line, then scratch
-    int16_t* es = el + Z * NKX;
-    if constexpr (sizeof(T) == 8) {
-        for (int e = threadIdx.x; e < N; e += blockDim.x) twx[e] = make_fxw(a.twg[e]);
-    } else {
-        for (int e = threadIdx.x; e < N; e += blockDim.x) tw[e] = a.twg[e];
-    }
+    for (int e = threadIdx.x; e < N; e += blockDim.x) twx[e] = make_fxw(a.twg[e]);
     for (int zz0 = 0; zz0 < Z; zz0 += ZB) {
-        if constexpr (sizeof(T) == 4) {
-            // four consecutive x per thread: 16-byte loads of the history, ds*w
-            // and Theta planes (N is a multiple of 4).  The four shared stores
-            // go out in an order rotated by (t / 4) % 4, which spreads the
-            // lanes of a warp over all bank pairs.
-            for (int t = threadIdx.x; t < ZB * PB / 4; t += blockDim.x) {
-                const int q = t / (PB / 4), e = 4 * (t % (PB / 4));
-                const int p = e / N, x = e % N;
-                const size_t ra = ((size_t)(z0 + zz0 + q) * N + 2 * p) * N + x, rb = ra + N;
-                const float4 va = rhs_f32x4(a, (size_t)i * NR + ra, ra);
-                const float4 vb = rhs_f32x4(a, (size_t)i * NR + rb, rb);
-                C* zq = zb + (size_t)q * PBS + p * XR + x;
-                const int rot = (t >> 2) & 3;
-#pragma unroll
-                for (int s = 0; s < 4; ++s) {
-                    const int c = (s + rot) & 3;
-                    const float xa = c == 0 ? va.x : c == 1 ? va.y : c == 2 ? va.z : va.w;
-                    const float xb = c == 0 ? vb.x : c == 1 ? vb.y : c == 2 ? vb.z : vb.w;
-                    zq[c] = cmk<C>(xa, xb);
-                }
-            }
-        } else {
-            for (int t = threadIdx.x; t < ZB * PB; t += blockDim.x) {
-                const int q = t / PB, e = t % PB;
-                const int p = e / N, x = e % N;
-                const size_t ra = ((size_t)(z0 + zz0 + q) * N + 2 * p) * N + x, rb = ra + N;
-                const T va = rhs_value<T, NR>(a, (size_t)i * NR + ra, ra);
-                const T vb = rhs_value<T, NR>(a, (size_t)i * NR + rb, rb);
-                zb[(size_t)q * PBS + p * XR + x] = cmk<C>(va, vb);
-            }
+        for (int t = threadIdx.x; t < ZB * PB; t += blockDim.x) {
+            const int q = t / PB, e = t % PB;
+            const int p = e / N, x = e % N;
+            const size_t ra = ((size_t)(z0 + zz0 + q) * N + 2 * p) * N + x, rb = ra + N;
+            const T va = rhs_value<T, NR>(a, (size_t)i * NR + ra, ra);
+            const T vb = rhs_value<T, NR>(a, (size_t)i * NR + rb, rb);
+            zb[(size_t)q * PBS + p * XR + x] = cmk<C>(va, vb);
         }
         __syncthreads();
-        if constexpr (sizeof(T) == 8)
-            fwd_x_planes_fx<N, Z, ZB>(zb, reinterpret_cast<fxc*>(out), zz0, twx, es, el);
-        else
-            fwd_x_planes<T, N, Z, ZB>(zb, out, zz0, tw);
+        fwd_x_planes_fx<N, Z, ZB>(zb, reinterpret_cast<fxc*>(out), zz0, twx, es, el);
     }
-    if constexpr (sizeof(T) == 8)  // the half spectra hold twice their value: exponent - 1
-        fx_nat2perm<N, -1, true>(out, NKX * Z, NKX * Z, 1, twx, es, es, from_fixed([=](int line, int y) {
-                                     return el[(line % Z) * (N / 2) + (y >> 1)] - 1;
-                                 }));
-    else
-        y_planes<T, N, Z, -1>(out, tw);
+    // the half spectra hold twice their value: exponent - 1
+    fx_nat2perm<N, -1, true>(out, NKX * Z, NKX * Z, 1, twx, es, es, from_fixed([=](int line, int y) {
+                                 return el[(line % Z) * (N / 2) + (y >> 1)] - 1;
+                             }));
     store_phat<T, N, Z>(a, out, i, z0);
 }
 
 // ---------------------------------------------------------------- pass C
 __host__ __device__ constexpr int ilog2(int n) { return n > 1 ? 1 + ilog2(n / 2) : 0; }
-// what the y-FFTs of pass C leave: fixed-point numbers in the FP64 form
-template <typename T> struct KspaceElem { using t = float2; };
-template <> struct KspaceElem<double> { using t = fxc; };
 
-template <typename T, int N, bool B = false, int V = 0>
-__global__ void __launch_bounds__(512) ifft_xy(StepArgs<T> a0, const StepArgs<T>* __restrict__ batch) {
-    const StepArgs<T> a = pick_args<B>(a0, batch);
-    using C = typename cvec<T>::t;
+// element k of the packed row ra + i rb, from the half spectra of its two real
+// rows (element k at [k * Z]); the imaginary parts at kx = 0 and N/2 are
+// discarded (c2r)
+template <int N, typename K> __device__ __forceinline__ K hermitian_pair(const K* ra, const K* rb, int k, int Z) {
+    K xa, xb;
+    if (k <= N / 2) {
+        xa = ra[k * Z];
+        xb = rb[k * Z];
+        if (k == 0 || k == N / 2) {
+            xa.y = decltype(xa.y)(0.0);
+            xb.y = decltype(xb.y)(0.0);
+        }
+    } else {
+        xa = ra[(N - k) * Z];
+        xb = rb[(N - k) * Z];
+        xa.y = -xa.y;
+        xb.y = -xb.y;
+    }
+    return cmk<K>(xa.x - xb.y, xa.y + xb.x);
+}
+
+template <int N, int V = 0> __global__ void __launch_bounds__(512) ifft_xy(StepArgs<double> a) {
+    using T = double;
+    using C = double2;
     constexpr int Z = XyShape<T, N, V>::Z, ZB = XyShape<T, N, V>::ZB;
     constexpr int NKX = N / 2 + 1;
     constexpr int NR = N * N * N;
@@ -263,39 +217,26 @@ __global__ void __launch_bounds__(512) ifft_xy(StepArgs<T> a0, const StepArgs<T>
     constexpr int XR = xrow(N), PBS = xplane(N);
     static_assert(PBS % 2 == 0, "the half-spectrum buffer must stay 16-byte aligned");
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    C* tw = reinterpret_cast<C*>(smem_raw);
-    C* zb = tw + N;                   // packed row pairs, row stride XR
+    fxw* twx = reinterpret_cast<fxw*>(smem_raw);
+    C* zb = reinterpret_cast<C*>(twx + N);  // packed row pairs, row stride XR
     C* out = zb + (size_t)ZB * PBS;
+    int16_t* el = reinterpret_cast<int16_t*>(out + (size_t)Z * N * NKX);  // exponents per line, then scratch
+    int16_t* es = el + Z * NKX;
     const int i = blockIdx.y;
     const int z0 = blockIdx.x * Z;
-    fxw* twx = reinterpret_cast<fxw*>(smem_raw);
-    int16_t* el = reinterpret_cast<int16_t*>(out + (size_t)Z * N * NKX);  // FP64 form: exponents per line, then scratch
-    int16_t* es = el + Z * NKX;
-    if constexpr (sizeof(T) == 8) {
-        for (int e = threadIdx.x; e < N; e += blockDim.x) twx[e] = make_fxw(a.twg[e]);
-    } else {
-        for (int e = threadIdx.x; e < N; e += blockDim.x) tw[e] = a.twg[e];
-    }
+    for (int e = threadIdx.x; e < N; e += blockDim.x) twx[e] = make_fxw(a.twg[e]);
     // 1/N^3 is a shift of the exponents where N is a power of two
-    constexpr bool kPow2 = sizeof(T) == 8 && (N & (N - 1)) == 0;
+    constexpr bool kPow2 = (N & (N - 1)) == 0;
     constexpr int kShift = kPow2 ? 3 * ilog2(N) : 0;
     // all loads issued up front: one Z-run (Z * sizeof(C) bytes) per (ky, kx)
-    constexpr int CH = (Z * (int)sizeof(C)) / 16;  // 16-byte chunks per run
-    static_assert((Z * sizeof(C)) % 16 == 0, "phat runs must be whole 16-byte chunks");
-    for (int e = threadIdx.x; e < N * NKX * CH; e += blockDim.x) {
-        const int col = e / CH, q = e % CH;
-        const C* src = a.phat + ((size_t)col * a.M + i) * N + z0;
-        cp_async16(reinterpret_cast<unsigned char*>(out + (size_t)col * Z) + 16 * q,
-                   reinterpret_cast<const unsigned char*>(src) + 16 * q);
+    for (int e = threadIdx.x; e < N * NKX * Z; e += blockDim.x) {
+        const int col = e / Z, q = e % Z;
+        cp_async16(out + (size_t)col * Z + q, a.phat + ((size_t)col * a.M + i) * N + z0 + q);
     }
-    cp_async_commit();
-    cp_async_wait<0>();
+    cp_async_wait_all();
     __syncthreads();
     // along y for every plane; row y now at perm_pos(y)
-    if constexpr (sizeof(T) == 8)
-        fx_nat2perm<N, +1, false>(out, NKX * Z, NKX * Z, 1, twx, es, el, FromDoubles{});
-    else
-        y_planes<T, N, Z, +1>(out, tw);
+    fx_nat2perm<N, +1, false>(out, NKX * Z, NKX * Z, 1, twx, es, el, FromDoubles{});
     for (int zz0 = 0; zz0 < Z; zz0 += ZB) {
         // Hermitian extension of rows (2p, 2p+1) packed as one complex row;
         // the imaginary parts at kx = 0 and N/2 are discarded (c2r)
@@ -305,33 +246,15 @@ __global__ void __launch_bounds__(512) ifft_xy(StepArgs<T> a0, const StepArgs<T>
             const int q = t % ZB, e = t / ZB;
             const int zz = zz0 + q;
             const int p = e / N, k = e % N;
-            using K = typename KspaceElem<T>::t;
-            const K* ra = reinterpret_cast<const K*>(out) + (size_t)perm_pos<N>(2 * p) * NKX * Z + zz;
-            const K* rb = reinterpret_cast<const K*>(out) + (size_t)perm_pos<N>(2 * p + 1) * NKX * Z + zz;
-            K xa, xb;
-            if (k <= N / 2) {
-                xa = ra[k * Z];
-                xb = rb[k * Z];
-                if (k == 0 || k == N / 2) {
-                    xa.y = decltype(xa.y)(0.0);
-                    xb.y = decltype(xb.y)(0.0);
-                }
-            } else {
-                xa = ra[(N - k) * Z];
-                xb = rb[(N - k) * Z];
-                xa.y = -xa.y;
-                xb.y = -xb.y;
-            }
-            reinterpret_cast<K*>(zb)[(size_t)q * PBS + p * XR + k] = cmk<K>(xa.x - xb.y, xa.y + xb.x);
+            const fxc* ra = reinterpret_cast<const fxc*>(out) + (size_t)perm_pos<N>(2 * p) * NKX * Z + zz;
+            const fxc* rb = reinterpret_cast<const fxc*>(out) + (size_t)perm_pos<N>(2 * p + 1) * NKX * Z + zz;
+            reinterpret_cast<fxc*>(zb)[(size_t)q * PBS + p * XR + k] = hermitian_pair<N>(ra, rb, k, Z);
         }
         __syncthreads();
         // along x; x at perm_pos(x)
-        if constexpr (sizeof(T) == 8)
-            fx_nat2perm<N, +1, true>(zb, ZB * (N / 2), 1, XR, twx, es, es, from_fixed([=](int line, int k) {
-                                         return el[(k <= N / 2 ? k : N - k) * Z + zz0 + line / (N / 2)] - kShift;
-                                     }));
-        else
-            fft_nat2perm<N, +1>(zb, ZB * (N / 2), 1, XR, tw);
+        fx_nat2perm<N, +1, true>(zb, ZB * (N / 2), 1, XR, twx, es, es, from_fixed([=](int line, int k) {
+                                     return el[(k <= N / 2 ? k : N - k) * Z + zz0 + line / (N / 2)] - kShift;
+                                 }));
         // packed row pair p holds rows 2p (real part) and 2p+1 (imaginary part)
         for (int t = threadIdx.x; t < ZB * PB; t += blockDim.x) {
             const int q = t / PB, e = t % PB;
@@ -352,6 +275,217 @@ __global__ void __launch_bounds__(512) ifft_xy(StepArgs<T> a0, const StepArgs<T>
     }
 }
 
+// ------------------------------------------------ FP32 form: passes A and C
+// The split of a packed row pair into its two half spectra (pass A) and the
+// Hermitian extension (pass C) happen in the loads of the next direction's
+// first sub-pass, and the last sub-pass writes to global memory: 9 and 8
+// shared-memory accesses of 8 bytes per complex point (12 with separate
+// split, pack and copy-out loops), which with the barriers between them bound
+// both passes.  A length N = R J is done as J transforms of length R over
+// elements n J + j (twiddle w^(j k)), then R transforms of length J over j.
+// Loading pass A's right-hand side straight into the first sub-pass was not
+// faster (32-byte pieces cost the L1 tags four times the 16-byte vectors').
+// 64^3, L = 10: pass A 171 -> 147 us, pass C 109 -> 89 us; 128^3, L = 12: 2.65 ->
+// 2.42 and 1.70 -> 1.23 ms; 24^3, L = 8: 14.0 -> 11.1 and 12.2 -> 9.7 us.
+
+// x lines.  Pass A: in place, element (n, j) and output n + R j at slot n S + j,
+// R = N2, so that 16-byte vectors of a row stay together (J >= 8).  Pass C:
+// slot (j, k) at j S + k, R = N1, so that neighbouring lanes write >= 4
+// neighbours of a row.  S odd: neighbouring lanes on distinct banks.
+template <int N, bool FWD> struct XLine {
+    static constexpr int R = FWD ? Plan<N>::N2 : Plan<N>::N1, J = N / R;
+    static constexpr int S = (FWD ? J : R) | 1;
+    static constexpr int ROW = (FWD ? R : J) * S;
+    __device__ __forceinline__ static int out_at(int k) { return (k % R) * S + k / R; }  // pass A, output k
+};
+template <int N> __host__ __device__ constexpr int xrow32(bool fwd) {
+    const int n1 = Plan<N>::N1, n2 = Plan<N>::N2;  // J of pass A and R of pass C are both N1
+    return fwd ? n2 * (n1 | 1) : n2 * (n1 | 1);
+}
+template <int N> __host__ __device__ constexpr int xrow32() {
+    return xrow32<N>(true) > xrow32<N>(false) ? xrow32<N>(true) : xrow32<N>(false);
+}
+__host__ inline int xrow32_of(int N) {
+    switch (N) {
+#define WLC_CASE(n) \
+    case n:         \
+        return xrow32<n>();
+        WLC_FOR_EACH_N(WLC_CASE)
+#undef WLC_CASE
+        default:
+            return 0;
+    }
+}
+
+template <int R, int DIR> __device__ __forceinline__ void twiddles(float2* v, int j, const float2* tw) {
+#pragma unroll
+    for (int k = 1; k < R; ++k)
+        if (j != 0) v[k] = cmul(v[k], twid<DIR>(tw, j * k));
+}
+
+// second sub-pass of the y lines in place, f(line, ky, value) for every output
+template <int N, int DIR, int Z, typename F> __device__ __forceinline__ void y_second(float2* out, F&& f) {
+    constexpr int NKX = N / 2 + 1, LS = NKX * Z, R = Plan<N>::N1, J = Plan<N>::N2;
+    for (LineWalk it(LS); it.j < R; it.next()) {
+        float2 v[J];
+#pragma unroll
+        for (int j = 0; j < J; ++j) v[j] = out[(j * R + it.j) * LS + it.b];
+        Dft<J>::template run<DIR>(v);
+#pragma unroll
+        for (int k2 = 0; k2 < J; ++k2) f(it.b, it.j + R * k2, v[k2]);
+    }
+}
+
+template <int N, bool B = false, int V = 0>
+__global__ void __launch_bounds__(512) rhs_fft_xy32(StepArgs<float> a0, const StepArgs<float>* __restrict__ batch) {
+    const StepArgs<float> a = pick_args<B>(a0, batch);
+    constexpr int Z = XyShape<float, N, V>::Z, ZB = XyShape<float, N, V>::ZB;
+    constexpr int NKX = N / 2 + 1, LS = NKX * Z, NR = N * N * N;
+    using X = XLine<N, true>;
+    constexpr int R = X::R, J = X::J, YR = Plan<N>::N1, YJ = Plan<N>::N2;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float2* tw = reinterpret_cast<float2*>(smem_raw);
+    float2* zb = tw + N;                             // [ZB][N/2] packed row pairs, X::ROW each
+    float2* out = zb + (size_t)ZB * (N / 2) * X::ROW;  // [N][NKX][Z]
+    const int i = blockIdx.y, z0 = blockIdx.x * Z;
+    for (int e = threadIdx.x; e < N; e += blockDim.x) tw[e] = a.twg[e];
+    __syncthreads();
+    for (int zz0 = 0; zz0 < Z; zz0 += ZB) {
+        // four consecutive x per thread: 16-byte loads of the history, ds*w and
+        // Theta planes; the four shared stores go out in an order rotated by
+        // lane, which spreads a warp over the banks
+        for (int t = threadIdx.x; t < ZB * (N / 2) * (N / 4); t += blockDim.x) {
+            const int b = t / (N / 4), x = 4 * (t % (N / 4));  // b = q N/2 + p
+            const size_t ra = ((size_t)(z0 + zz0 + b / (N / 2)) * N + 2 * (b % (N / 2))) * N + x, rb = ra + N;
+            const float4 va = rhs_f32x4(a, (size_t)i * NR + ra, ra);
+            const float4 vb = rhs_f32x4(a, (size_t)i * NR + rb, rb);
+            float2* zq = zb + (size_t)b * X::ROW + (x / J) * X::S + x % J;
+            const int rot = (t >> 2) & 3;
+#pragma unroll
+            for (int s = 0; s < 4; ++s) {
+                const int c = (s + rot) & 3;
+                zq[c] = make_float2(c == 0 ? va.x : c == 1 ? va.y : c == 2 ? va.z : va.w,
+                                    c == 0 ? vb.x : c == 1 ? vb.y : c == 2 ? vb.z : vb.w);
+            }
+        }
+        __syncthreads();
+        if constexpr (R > 1) {
+            for (int w = threadIdx.x; w < ZB * (N / 2) * J; w += blockDim.x) {
+                const int j = w % J;
+                float2* row = zb + (size_t)(w / J) * X::ROW + j;
+                float2 v[R];
+#pragma unroll
+                for (int n = 0; n < R; ++n) v[n] = row[n * X::S];
+                Dft<R>::template run<-1>(v);
+                twiddles<R, -1>(v, j, tw);
+#pragma unroll
+                for (int n = 0; n < R; ++n) row[n * X::S] = v[n];
+            }
+            __syncthreads();
+        }
+        for (int w = threadIdx.x; w < ZB * (N / 2) * R; w += blockDim.x) {
+            float2* row = zb + (size_t)(w / R) * X::ROW + (w % R) * X::S;
+            float2 v[J];
+#pragma unroll
+            for (int j = 0; j < J; ++j) v[j] = row[j];
+            Dft<J>::template run<-1>(v);
+#pragma unroll
+            for (int j = 0; j < J; ++j) row[j] = v[j];
+        }
+        __syncthreads();
+        // first y sub-pass on the half spectra of rows (2p, 2p+1): lines (kx, plane)
+        for (LineWalk it(NKX * ZB); it.j < YJ; it.next()) {
+            const int q = it.b % ZB, kx = it.b / ZB;
+            const float2* zk = zb + (size_t)q * (N / 2) * X::ROW + X::out_at(kx);
+            const float2* zm = zb + (size_t)q * (N / 2) * X::ROW + X::out_at((N - kx) % N);
+            float2 v[YR];
+#pragma unroll
+            for (int n = 0; n < YR; ++n) {
+                const int y = n * YJ + it.j;
+                const float2 c = zk[(y >> 1) * X::ROW], d = zm[(y >> 1) * X::ROW];
+                v[n] = (y & 1) ? make_float2(0.5f * (c.y + d.y), 0.5f * (d.x - c.x))
+                               : make_float2(0.5f * (c.x + d.x), 0.5f * (c.y - d.y));
+            }
+            Dft<YR>::template run<-1>(v);
+            twiddles<YR, -1>(v, it.j, tw);
+            float2* o = out + (size_t)it.j * YR * LS + kx * Z + zz0 + q;
+#pragma unroll
+            for (int k = 0; k < YR; ++k) o[k * LS] = v[k];
+        }
+        __syncthreads();
+    }
+    y_second<N, -1, Z>(out, [&](int b, int ky, float2 v) {
+        a.phat[((size_t)(ky * NKX + b / Z) * a.M + i) * N + z0 + b % Z] = v;
+    });
+}
+
+template <int N, bool B = false, int V = 0>
+__global__ void __launch_bounds__(512) ifft_xy32(StepArgs<float> a0, const StepArgs<float>* __restrict__ batch) {
+    const StepArgs<float> a = pick_args<B>(a0, batch);
+    constexpr int Z = XyShape<float, N, V>::Z, ZB = XyShape<float, N, V>::ZB;
+    constexpr int NKX = N / 2 + 1, LS = NKX * Z, NR = N * N * N;
+    using X = XLine<N, false>;
+    constexpr int R = X::R, J = X::J;
+    static_assert(X::ROW * (N / 2) % 2 == 0, "the half-spectrum buffer must stay 16-byte aligned");
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float2* tw = reinterpret_cast<float2*>(smem_raw);
+    float2* zb = tw + N;
+    float2* out = zb + (size_t)ZB * (N / 2) * X::ROW;
+    const int i = blockIdx.y, z0 = blockIdx.x * Z;
+    for (int e = threadIdx.x; e < N; e += blockDim.x) tw[e] = a.twg[e];
+    __syncthreads();
+    // all loads issued up front: one Z-run (8 Z bytes) per (ky, kx)
+    constexpr int CH = Z / 2;  // 16-byte chunks per run
+    static_assert(Z % 2 == 0, "phat runs must be whole 16-byte chunks");
+    for (int e = threadIdx.x; e < N * NKX * CH; e += blockDim.x) {
+        const int col = e / CH, q = e % CH;
+        cp_async16(out + (size_t)col * Z + 2 * q, a.phat + ((size_t)col * a.M + i) * N + z0 + 2 * q);
+    }
+    cp_async_wait_all();
+    __syncthreads();
+    fft_nat2perm<N, +1>(out, LS, LS, 1, tw);  // along y for every plane; row y now at perm_pos(y)
+    for (int zz0 = 0; zz0 < Z; zz0 += ZB) {
+        // Hermitian extension of rows (2p, 2p+1) packed as one complex row
+        for (int w = threadIdx.x; w < ZB * (N / 2) * J; w += blockDim.x) {
+            // plane fastest across the lanes, then j: neighbours in out
+            const int q = w % ZB, j = w / ZB % J, p = w / (ZB * J), b = q * (N / 2) + p;
+            const float2* ra = out + (size_t)perm_pos<N>(2 * p) * LS + zz0 + q;
+            const float2* rb = out + (size_t)perm_pos<N>(2 * p + 1) * LS + zz0 + q;
+            float2 v[R];
+#pragma unroll
+            for (int n = 0; n < R; ++n) v[n] = hermitian_pair<N>(ra, rb, n * J + j, Z);
+            Dft<R>::template run<+1>(v);
+            twiddles<R, +1>(v, j, tw);
+            float2* row = zb + (size_t)b * X::ROW + j * X::S;
+#pragma unroll
+            for (int k = 0; k < R; ++k) row[k] = v[k];
+        }
+        __syncthreads();
+        // packed row pair p holds rows 2p (real part) and 2p+1 (imaginary part)
+        for (int w = threadIdx.x; w < ZB * (N / 2) * R; w += blockDim.x) {
+            const int k = w % R, b = w / R;
+            const float2* row = zb + (size_t)b * X::ROW + k;
+            float2 v[J];
+#pragma unroll
+            for (int j = 0; j < J; ++j) v[j] = row[j * X::S];
+            Dft<J>::template run<+1>(v);
+            const size_t r = ((size_t)(z0 + zz0 + b / (N / 2)) * N + 2 * (b % (N / 2))) * N + k;
+            float* dst = a.qout + (size_t)i * NR + r;
+#pragma unroll
+            for (int j = 0; j < J; ++j) {
+                float2 u = cscale(v[j], a.minv);
+                if (a.post) {  // split scheme: the second field half step
+                    u.x *= a.post[r + R * j];
+                    u.y *= a.post[r + R * j + N];
+                }
+                dst[R * j] = u.x;
+                dst[R * j + N] = u.y;
+            }
+        }
+        __syncthreads();
+    }
+}
+
 // right-hand side only (init_pr test hook), out[i][r]
 template <typename T, int N>
 __global__ void __launch_bounds__(256) rhs_only(StepArgs<T> a, T* out) {
@@ -365,51 +499,49 @@ __global__ void __launch_bounds__(256) rhs_only(StepArgs<T> a, T* out) {
 template <typename T> size_t smem_xy(int N, int variant) {
     using C = typename cvec<T>::t;
     const int z = xy_planes(N, sizeof(T), variant & 1), zb = (variant & 2) ? z : 1;
-    return sizeof(C) * ((size_t)N + (size_t)zb * xplane(N) + (size_t)z * N * (N / 2 + 1)) +
+    const size_t plane = sizeof(T) == 8 ? (size_t)xplane(N) : (size_t)(N / 2) * xrow32_of(N);
+    return sizeof(C) * ((size_t)N + zb * plane + (size_t)z * N * (N / 2 + 1)) +
            (sizeof(T) == 8 ? 2 * (size_t)xy_exps(N, z, zb) : 0);
 }
 
 // shared-memory limits of the pass A / pass C kernels of (T, N, B), once per
 // (kernel, device); returns the first error
+template <typename T, int N, bool B, int V> static const void* xy_kernel(bool do_a) {
+    if constexpr (sizeof(T) == 4)
+        return do_a ? (const void*)rhs_fft_xy32<N, B, V> : (const void*)ifft_xy32<N, B, V>;
+    else
+        return do_a ? (const void*)rhs_fft_xy<N, V> : (const void*)ifft_xy<N, V>;
+}
+constexpr int kXySmem = 220 * 1024;
 template <typename T, int N, bool B> static cudaError_t set_xy_attrs() {
-    constexpr int big = 200 * 1024;
     cudaError_t e = cudaSuccess;
-    auto set = [&](const void* fn, int bytes) {
-        const cudaError_t r = smem_attr_once(fn, bytes);
-        if (e == cudaSuccess) e = r;
+    auto set = [&](const void* a, const void* c) {
+        for (const void* fn : {a, c}) {
+            const cudaError_t r = smem_attr_once(fn, kXySmem);
+            if (e == cudaSuccess) e = r;
+        }
     };
-    set((const void*)rhs_fft_xy<T, N, B, 0>, big);
-    set((const void*)ifft_xy<T, N, B, 0>, big);
-    set((const void*)rhs_fft_xy<T, N, B, 1>, big);
-    set((const void*)ifft_xy<T, N, B, 1>, big);
-    if (smem_xy<T>(N, 2) <= (size_t)big) {
-        set((const void*)rhs_fft_xy<T, N, B, 2>, big);
-        set((const void*)ifft_xy<T, N, B, 2>, big);
-    }
-    if (smem_xy<T>(N, 3) <= (size_t)big) {
-        set((const void*)rhs_fft_xy<T, N, B, 3>, big);
-        set((const void*)ifft_xy<T, N, B, 3>, big);
-    }
+    set(xy_kernel<T, N, B, 0>(true), xy_kernel<T, N, B, 0>(false));
+    set(xy_kernel<T, N, B, 1>(true), xy_kernel<T, N, B, 1>(false));
+    set(xy_kernel<T, N, B, 2>(true), xy_kernel<T, N, B, 2>(false));
+    set(xy_kernel<T, N, B, 3>(true), xy_kernel<T, N, B, 3>(false));
     return e;
 }
 
-// Launch shape of passes A and C when none is set (threads = variant = 0),
-// by the CTAs that fit an SM's shared memory.  FP32: the batched x-FFTs on
-// half planes (variant 3: fewest barriers and still several CTAs), unless
-// that leaves one CTA; 256 threads from 4 CTAs on, else 512.  FP64: whole
-// planes with batched x-FFTs while 4 CTAs fit (twice the work per barrier),
-// else half planes; 512 threads for a lone CTA.  Measured per step (us,
-// 256-thread variant 0 -> this): FP32 pass A 24^3 16 -> 14, 48^3 70 -> 56,
-// 64^3 189 -> 171, 128^3 3570 -> 2650; pass C 64^3 135 -> 109, 128^3 1956 ->
-// 1695; FP64 pass A 40^3 120 -> 112, 64^3 655 -> 527, pass C 24^3 22 -> 15.
+// Launch shape of passes A and C when none is set (threads = variant = 0), by
+// the CTAs that fit an SM's shared memory: whole planes with all x-FFTs in one
+// batched call (variant 2, the most work per barrier) with 256 threads while 4
+// CTAs fit, else half planes and one plane's x-FFTs at a time (variant 1, the
+// smallest CTAs), with 512 threads where few of those fit.  Measured (us per
+// step, the next best of the other seven shapes in brackets): FP32 pass A 24^3
+// 11.1 (12.3), 48^3 53.8 (54.3), 64^3 147 (143, but 4 more in pass C), 96^3 436
+// (507); pass C 40^3 18.9 (20.9), 64^3 88.6 (90.2), 96^3 228 (247); FP64 pass
+// A 40^3 112 (120), 64^3 527 (655); pass C 24^3 14.6 (18.7).
 template <typename T> static void xy_shape(int N, int& threads, int& variant) {
     if (threads == 0 && variant == 0) {
         auto ctas = [&](int v) { return (int)(227 * 1024 / (smem_xy<T>(N, v) + 1024)); };
-        if (sizeof(T) == 4)
-            variant = ctas(3) >= 2 ? 3 : 1;
-        else
-            variant = ctas(2) >= 4 ? 2 : 1;
-        threads = ctas(variant) >= (sizeof(T) == 4 ? 4 : 2) ? 256 : 512;
+        variant = ctas(2) >= 4 ? 2 : 1;
+        threads = variant == 2 || ctas(1) >= (sizeof(T) == 4 ? 5 : 2) ? 256 : 512;
     }
     threads = threads == 512 ? 512 : 256;
 }
@@ -422,17 +554,24 @@ static void launch_xy(bool do_a, const StepArgs<T>& a, const StepArgs<T>* batch,
     constexpr int Z = XyShape<T, N, V>::Z;
     const size_t sxy = smem_xy<T>(N, V);
     const dim3 g(N / Z, M, count);
-    if (do_a)
-        rhs_fft_xy<T, N, B, V><<<g, threads, sxy, st>>>(a, batch);
-    else
-        ifft_xy<T, N, B, V><<<g, threads, sxy, st>>>(a, batch);
+    if constexpr (sizeof(T) == 4) {
+        if (do_a)
+            rhs_fft_xy32<N, B, V><<<g, threads, sxy, st>>>(a, batch);
+        else
+            ifft_xy32<N, B, V><<<g, threads, sxy, st>>>(a, batch);
+    } else {
+        if (do_a)
+            rhs_fft_xy<N, V><<<g, threads, sxy, st>>>(a);
+        else
+            ifft_xy<N, V><<<g, threads, sxy, st>>>(a);
+    }
 }
 
 template <typename T, int N, bool B>
 static void launch_xy_any(int variant, bool do_a, const StepArgs<T>& a, const StepArgs<T>* batch, int M, int count,
                           int threads, cudaStream_t st) {
     xy_shape<T>(N, threads, variant);
-    if ((variant & 2) && smem_xy<T>(N, variant) > 200 * 1024) variant &= 1;  // batched x-FFTs do not fit
+    if ((variant & 2) && smem_xy<T>(N, variant) > kXySmem) variant &= 1;  // batched x-FFTs do not fit
     switch (variant & 3) {
         case 1: launch_xy<T, N, B, 1>(do_a, a, batch, M, count, threads, st); break;
         case 2: launch_xy<T, N, B, 2>(do_a, a, batch, M, count, threads, st); break;
