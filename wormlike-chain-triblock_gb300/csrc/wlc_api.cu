@@ -761,17 +761,18 @@ extern "C" int wlc_density(wlc_ctx* c, double* phi, double* junc, double* s_op, 
         c->launches++;
     }
     if (s_op) {
-        std::vector<double> h(15 * nr);
-        CK(cudaMemcpyAsync(h.data(), c->srs, sizeof(double) * 15 * nr, cudaMemcpyDeviceToHost, c->st));
+        // S_OP_blk(r, a, b, blk) at s_op[r + nr*(a + 3b + 9 blk)], written out
+        // from the five components on the device, as many planes at a time as
+        // the transfer buffer (M planes) holds
+        const int64_t hold = std::min<int64_t>(27, c->M);
+        for (int p0 = 0; p0 < 27; p0 += (int)hold) {
+            const int np = (int)std::min<int64_t>(hold, 27 - p0);
+            launch_s_planes(c->srs, c->stage, p0, np, c->nr, c->st);
+            c->launches++;
+            CK(cudaMemcpyAsync(s_op + (size_t)p0 * nr, c->stage, sizeof(double) * (size_t)np * nr, cudaMemcpyDeviceToHost,
+                               c->st));
+        }
         CK(cudaStreamSynchronize(c->st));
-        // S_OP_blk(r, a, b, blk) at s_op[r + nr*(a + 3b + 9 blk)]; S_zz = -S_xx - S_yy
-        for (int b = 0; b < 3; ++b)
-            for (size_t r = 0; r < nr; ++r) {
-                const double* t = h.data() + (size_t)b * 5 * nr + r;
-                const double sxx = t[0], syy = t[nr], sxy = t[2 * nr], sxz = t[3 * nr], syz = t[4 * nr];
-                const double S[9] = {sxx, sxy, sxz, sxy, syy, syz, sxz, syz, -(sxx + syy)};
-                for (int q = 0; q < 9; ++q) s_op[r + nr * (q + 9 * (size_t)b)] = S[q];
-            }
     }
     c->have_density = true;
     return WLC_OK;

@@ -8,6 +8,7 @@
 //
 // All reductions are deterministic: fixed partition per CTA, fixed-order
 // tree in shared memory, one final CTA summing the partials in order.
+#include <algorithm>
 #include <cstdint>
 
 #include "wlc_attr.h"
@@ -672,6 +673,18 @@ __global__ void fe_integrand(const double* __restrict__ phi, const double* __res
     }
 }
 
+// One read and one write per value; expanding on the host took 40 ms of a
+// 128^3 call (27 planes of 2 M points), the transfer itself 20 ms.
+__global__ void s_planes(const double* __restrict__ s, double* __restrict__ out, int p0, int64_t nr) {
+    const int p = p0 + blockIdx.y, b = p / 9, q = p % 9;
+    const int8_t comp[9] = {0, 2, 3, 2, 1, 4, 3, 4, -1};
+    const double* c = s + (int64_t)b * 5 * nr;
+    double* o = out + (int64_t)blockIdx.y * nr;
+    const int k = comp[q];
+    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < nr; r += (int64_t)gridDim.x * blockDim.x)
+        o[r] = k >= 0 ? c[k * nr + r] : -(c[r] + c[nr + r]);
+}
+
 __global__ void count_nonfinite(const double* __restrict__ a, int64_t n, int* __restrict__ flag) {
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x)
         if (!isfinite(a[e])) atomicOr(flag, 1);
@@ -756,6 +769,10 @@ void launch_scale(double* a, int64_t n, const double* denom, double vol, cudaStr
 
 void launch_fe(const double* phi, const double* w, const double* mop, const FeArgs& f, double* ar, cudaStream_t st) {
     fe_integrand<<<grid_for(f.nr), 256, 0, st>>>(phi, w, mop, f, ar);
+}
+
+void launch_s_planes(const double* s, double* out, int p0, int np, int64_t nr, cudaStream_t st) {
+    s_planes<<<dim3(std::min(grid_for(nr), 512), np), 256, 0, st>>>(s, out, p0, nr);
 }
 
 void launch_nonfinite(const double* a, int64_t n, int* flag, cudaStream_t st) {

@@ -99,6 +99,9 @@ void launch_s3(const double* a, int nsum, int64_t stride, const S3Args& s, doubl
                cudaStream_t st);
 void launch_scale(double* a, int64_t n, const double* denom, double vol, cudaStream_t st);
 void launch_fe(const double* phi, const double* w, const double* mop, const FeArgs& f, double* ar, cudaStream_t st);
+// planes p0 .. p0+np-1 of S_OP(r, a, b, blk) (plane a + 3b + 9 blk) from the
+// components s[blk][5][nr] (xx, yy, xy, xz, yz); S_zz = -(S_xx + S_yy)
+void launch_s_planes(const double* s, double* out, int p0, int np, int64_t nr, cudaStream_t st);
 void launch_nonfinite(const double* a, int64_t n, int* flag, cudaStream_t st);
 
 }  // namespace wlc
