@@ -36,4 +36,41 @@ template <typename K> inline cudaError_t smem_attr_once(K* fn, int bytes) {
     return smem_attr_once(reinterpret_cast<const void*>(fn), bytes);
 }
 
+// Launch of a kernel that begins with dep_wait() below: with `chain` it may be
+// put in place while the kernel before it on the stream finishes (programmatic
+// dependent launch), which takes the launch latency between the passes of a
+// contour step off their chain.  chained_step: where that was faster -- short
+// kernels (iterations at 16^3, L = 2 FP64 4.87 -> 4.33 ms, 40^3, L = 7 FP32 10.6 ->
+// 9.85 ms); CTAs put in place early hold shared memory that the other sweep's
+// kernels could use (32^3, L = 6 FP64 27.2 -> 28.7 ms, 64^3 FP32 98.5 -> 99.4 ms).
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+constexpr bool chained_step(int N, int tsize, bool batched) { return !batched && N <= (tsize == 4 ? 48 : 24); }
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(bool chain, void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t st,
+                                  A... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = chain ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+#ifdef __CUDACC__
+// every kernel before this one on the stream has finished and its writes are visible
+template <bool CHAINED> __device__ __forceinline__ void dep_wait() {
+    if constexpr (CHAINED) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// the next kernel on the stream may be put in place once every CTA has come here
+template <bool CHAINED> __device__ __forceinline__ void dep_next() {
+    if constexpr (CHAINED) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+#endif
+
 }  // namespace wlc

@@ -251,6 +251,7 @@ extern "C" int wlc_mde_one_step_noalloc(const wlc_params* p, int32_t g_index, co
     ds.phat = reinterpret_cast<double2*>(ds.base + phat_off);
 
     StepLaunch<double> Lh;
+    Lh.chain_a = false;  // what precedes it on the caller's stream, or in its capture, is the caller's
     StepArgs<double>& a = Lh.step;
     a.h1 = pr_dev;
     a.h2 = nullptr;

@@ -361,6 +361,7 @@ __global__ void __maxnreg__(sizeof(T) == 4 ? 80 : 128)
     float2* corr = reinterpret_cast<float2*>(smem_raw + sm.corr);
     const int colid = blockIdx.x;
     C* gcol = a.phat + (size_t)colid * M * N;
+    dep_wait<chained_step(N, sizeof(T), B)>();
     for (int e = threadIdx.x; e < M * N; e += blockDim.x) cp_async_elem(col + (e / N) * NP + (e % N), gcol + e);
     asm volatile("cp.async.commit_group;\n" ::: "memory");
     stage(s_zoff, g.zoff, M);
@@ -553,6 +554,7 @@ __global__ void __maxnreg__(sizeof(T) == 4 ? 80 : 128)
             fx_perm2nat<N, +1, true>(col, M, 1, NP, twx, es, es, FromDoubles{});
     } else
         fft_perm2nat<N, +1>(col, M, 1, NP, tw);
+    dep_next<chained_step(N, sizeof(T), B)>();
     if (a.split) {
         // Crank-Nicolson operator (I + ds/2 A)^-1 (I - ds/2 A) = 2 (I + ds/2 A)^-1 - I
         // applied through the z transforms: IFFT_z(2x - b) = 2 IFFT_z(x) - N b,
@@ -652,8 +654,8 @@ template <typename T, int N> static cudaError_t launch_solve_n(const SolveArgs<T
     if (const cudaError_t e = smem_attr_once((const void*)zfft_solve<T, N>, 227 * 1024); e != cudaSuccess) return e;
     const size_t smem = solve_smem_bytes<T>(a);
     const int parts = solve_parts<T>(N, a.tab.L, threads, smem, a.nkx * N);
-    zfft_solve<T, N><<<a.nkx * N, 2 * N * parts, smem, st>>>(a, nullptr, solve_split(a.tab.L, parts));
-    return cudaGetLastError();
+    return launch_chained(chained_step(N, sizeof(T), false), zfft_solve<T, N>, dim3(a.nkx * N), 2 * N * parts, smem, st, a, nullptr,
+                          solve_split(a.tab.L, parts));
 }
 
 template <typename T> cudaError_t launch_solve(int N, const SolveArgs<T>& a, cudaStream_t st, int threads) {
@@ -675,9 +677,8 @@ template <int N> static cudaError_t set_solve_batched_attr() {
 template <int N> static cudaError_t launch_solve_batched_n(const BatchLaunch<float>& b, cudaStream_t st) {
     if (const cudaError_t e = set_solve_batched_attr<N>(); e != cudaSuccess) return e;
     const int parts = solve_parts<float>(N, b.lmax, b.solve_threads, b.solve_smem, b.nkx * N * b.count);
-    zfft_solve<float, N, true><<<dim3(b.nkx * N, 1, b.count), 2 * N * parts, b.solve_smem, st>>>(
-        SolveArgs<float>{}, b.dsolve, solve_split(b.lmax, parts));
-    return cudaGetLastError();
+    return launch_chained(chained_step(N, 4, true), zfft_solve<float, N, true>, dim3(b.nkx * N, 1, b.count), 2 * N * parts, b.solve_smem, st,
+                          SolveArgs<float>{}, b.dsolve, solve_split(b.lmax, parts));
 }
 
 cudaError_t launch_solve_batched(int N, const BatchLaunch<float>& b, cudaStream_t st) {

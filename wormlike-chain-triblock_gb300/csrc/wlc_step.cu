@@ -164,6 +164,7 @@ __global__ void __launch_bounds__(512) rhs_fft_xy(StepArgs<double> a) {
     const int i = blockIdx.y;
     const int z0 = blockIdx.x * Z;
     for (int e = threadIdx.x; e < N; e += blockDim.x) twx[e] = make_fxw(a.twg[e]);
+    dep_wait<chained_step(N, 8, false)>();
     for (int zz0 = 0; zz0 < Z; zz0 += ZB) {
         for (int t = threadIdx.x; t < ZB * PB; t += blockDim.x) {
             const int q = t / PB, e = t % PB;
@@ -180,6 +181,7 @@ __global__ void __launch_bounds__(512) rhs_fft_xy(StepArgs<double> a) {
     fx_nat2perm<N, -1, true>(out, NKX * Z, NKX * Z, 1, twx, es, es, from_fixed([=](int line, int y) {
                                  return el[(line % Z) * (N / 2) + (y >> 1)] - 1;
                              }));
+    dep_next<chained_step(N, 8, false)>();
     store_phat<T, N, Z>(a, out, i, z0);
 }
 
@@ -225,6 +227,7 @@ template <int N, int V = 0> __global__ void __launch_bounds__(512) ifft_xy(StepA
     const int i = blockIdx.y;
     const int z0 = blockIdx.x * Z;
     for (int e = threadIdx.x; e < N; e += blockDim.x) twx[e] = make_fxw(a.twg[e]);
+    dep_wait<chained_step(N, 8, false)>();
     // 1/N^3 is a shift of the exponents where N is a power of two
     constexpr bool kPow2 = (N & (N - 1)) == 0;
     constexpr int kShift = kPow2 ? 3 * ilog2(N) : 0;
@@ -255,6 +258,7 @@ template <int N, int V = 0> __global__ void __launch_bounds__(512) ifft_xy(StepA
         fx_nat2perm<N, +1, true>(zb, ZB * (N / 2), 1, XR, twx, es, es, from_fixed([=](int line, int k) {
                                      return el[(k <= N / 2 ? k : N - k) * Z + zz0 + line / (N / 2)] - kShift;
                                  }));
+        if (zz0 + ZB >= Z) dep_next<chained_step(N, 8, false)>();
         // packed row pair p holds rows 2p (real part) and 2p+1 (imaginary part)
         for (int t = threadIdx.x; t < ZB * PB; t += blockDim.x) {
             const int q = t / PB, e = t % PB;
@@ -349,6 +353,7 @@ __global__ void __launch_bounds__(512) rhs_fft_xy32(StepArgs<float> a0, const St
     float2* out = zb + (size_t)ZB * (N / 2) * X::ROW;  // [N][NKX][Z]
     const int i = blockIdx.y, z0 = blockIdx.x * Z;
     for (int e = threadIdx.x; e < N; e += blockDim.x) tw[e] = a.twg[e];
+    dep_wait<chained_step(N, 4, B)>();
     __syncthreads();
     for (int zz0 = 0; zz0 < Z; zz0 += ZB) {
         // four consecutive x per thread: 16-byte loads of the history, ds*w and
@@ -414,6 +419,7 @@ __global__ void __launch_bounds__(512) rhs_fft_xy32(StepArgs<float> a0, const St
         }
         __syncthreads();
     }
+    dep_next<chained_step(N, 4, B)>();
     y_second<N, -1, Z>(out, [&](int b, int ky, float2 v) {
         a.phat[((size_t)(ky * NKX + b / Z) * a.M + i) * N + z0 + b % Z] = v;
     });
@@ -433,6 +439,7 @@ __global__ void __launch_bounds__(512) ifft_xy32(StepArgs<float> a0, const StepA
     float2* out = zb + (size_t)ZB * (N / 2) * X::ROW;
     const int i = blockIdx.y, z0 = blockIdx.x * Z;
     for (int e = threadIdx.x; e < N; e += blockDim.x) tw[e] = a.twg[e];
+    dep_wait<chained_step(N, 4, B)>();
     __syncthreads();
     // all loads issued up front: one Z-run (8 Z bytes) per (ky, kx)
     constexpr int CH = Z / 2;  // 16-byte chunks per run
@@ -461,6 +468,7 @@ __global__ void __launch_bounds__(512) ifft_xy32(StepArgs<float> a0, const StepA
             for (int k = 0; k < R; ++k) row[k] = v[k];
         }
         __syncthreads();
+        if (zz0 + ZB >= Z) dep_next<chained_step(N, 4, B)>();
         // packed row pair p holds rows 2p (real part) and 2p+1 (imaginary part)
         for (int w = threadIdx.x; w < ZB * (N / 2) * R; w += blockDim.x) {
             const int k = w % R, b = w / R;
@@ -550,54 +558,54 @@ template <typename T> static void xy_shape(int N, int& threads, int& variant) {
 // batched x-FFTs)
 template <typename T, int N, bool B, int V>
 static void launch_xy(bool do_a, const StepArgs<T>& a, const StepArgs<T>* batch, int M, int count, int threads,
-                      cudaStream_t st) {
+                      bool chain, cudaStream_t st) {
     constexpr int Z = XyShape<T, N, V>::Z;
     const size_t sxy = smem_xy<T>(N, V);
     const dim3 g(N / Z, M, count);
     if constexpr (sizeof(T) == 4) {
         if (do_a)
-            rhs_fft_xy32<N, B, V><<<g, threads, sxy, st>>>(a, batch);
+            launch_chained(chain && chained_step(N, 4, B), rhs_fft_xy32<N, B, V>, g, threads, sxy, st, a, batch);
         else
-            ifft_xy32<N, B, V><<<g, threads, sxy, st>>>(a, batch);
+            launch_chained(chain && chained_step(N, 4, B), ifft_xy32<N, B, V>, g, threads, sxy, st, a, batch);
     } else {
         if (do_a)
-            rhs_fft_xy<N, V><<<g, threads, sxy, st>>>(a);
+            launch_chained(chain && chained_step(N, 8, B), rhs_fft_xy<N, V>, g, threads, sxy, st, a);
         else
-            ifft_xy<N, V><<<g, threads, sxy, st>>>(a);
+            launch_chained(chain && chained_step(N, 8, B), ifft_xy<N, V>, g, threads, sxy, st, a);
     }
 }
 
 template <typename T, int N, bool B>
 static void launch_xy_any(int variant, bool do_a, const StepArgs<T>& a, const StepArgs<T>* batch, int M, int count,
-                          int threads, cudaStream_t st) {
+                          int threads, bool chain, cudaStream_t st) {
     xy_shape<T>(N, threads, variant);
     if ((variant & 2) && smem_xy<T>(N, variant) > kXySmem) variant &= 1;  // batched x-FFTs do not fit
     switch (variant & 3) {
-        case 1: launch_xy<T, N, B, 1>(do_a, a, batch, M, count, threads, st); break;
-        case 2: launch_xy<T, N, B, 2>(do_a, a, batch, M, count, threads, st); break;
-        case 3: launch_xy<T, N, B, 3>(do_a, a, batch, M, count, threads, st); break;
-        default: launch_xy<T, N, B, 0>(do_a, a, batch, M, count, threads, st); break;
+        case 1: launch_xy<T, N, B, 1>(do_a, a, batch, M, count, threads, chain, st); break;
+        case 2: launch_xy<T, N, B, 2>(do_a, a, batch, M, count, threads, chain, st); break;
+        case 3: launch_xy<T, N, B, 3>(do_a, a, batch, M, count, threads, chain, st); break;
+        default: launch_xy<T, N, B, 0>(do_a, a, batch, M, count, threads, chain, st); break;
     }
 }
 
 template <typename T, int N> static cudaError_t launch_n(const StepLaunch<T>& s, cudaStream_t st) {
     if (const cudaError_t ea = set_xy_attrs<T, N, false>(); ea != cudaSuccess) return ea;
     if (s.events) cudaEventRecord(s.events[0], st);
-    if (s.do_a) launch_xy_any<T, N, false>(s.xy_z, true, s.step, nullptr, s.step.M, 1, s.xy_threads, st);
+    if (s.do_a) launch_xy_any<T, N, false>(s.xy_z, true, s.step, nullptr, s.step.M, 1, s.xy_threads, s.chain_a, st);
     if (s.events) cudaEventRecord(s.events[1], st);
     if (s.do_b) launch_solve<T>(N, s.solve, st, s.solve_threads);
     if (s.events) cudaEventRecord(s.events[2], st);
-    if (s.do_c) launch_xy_any<T, N, false>(s.xy_z, false, s.step, nullptr, s.step.M, 1, s.xy_threads, st);
+    if (s.do_c) launch_xy_any<T, N, false>(s.xy_z, false, s.step, nullptr, s.step.M, 1, s.xy_threads, true, st);
     if (s.events) cudaEventRecord(s.events[3], st);
     return cudaGetLastError();
 }
 
 template <int N> static cudaError_t launch_batched_n(const BatchLaunch<float>& b, cudaStream_t st) {
     if (const cudaError_t ea = set_xy_attrs<float, N, true>(); ea != cudaSuccess) return ea;
-    launch_xy_any<float, N, true>(b.xy_z, true, StepArgs<float>{}, b.dstep, b.M, b.count, b.xy_threads, st);
+    launch_xy_any<float, N, true>(b.xy_z, true, StepArgs<float>{}, b.dstep, b.M, b.count, b.xy_threads, false, st);
     cudaError_t e = launch_solve_batched(N, b, st);
     if (e != cudaSuccess) return e;
-    launch_xy_any<float, N, true>(b.xy_z, false, StepArgs<float>{}, b.dstep, b.M, b.count, b.xy_threads, st);
+    launch_xy_any<float, N, true>(b.xy_z, false, StepArgs<float>{}, b.dstep, b.M, b.count, b.xy_threads, false, st);
     return cudaGetLastError();
 }
 

@@ -15,6 +15,7 @@ template <typename T> struct StepLaunch {
     StepArgs<T> step;
     SolveArgs<T> solve;
     bool do_a = true, do_b = true, do_c = true;
+    bool chain_a = true;    // pass A may follow the work before it as a programmatic dependent (launch_chained)
     int solve_threads = 0;  // pass B threads per CTA (0: default)
     int xy_threads = 0;     // pass A and pass C threads per CTA (256 or 512)
     int xy_z = 0;           // pass A and pass C variant (bit 0 half planes, bit 1 batched x-FFTs); 0 and 0: by size
