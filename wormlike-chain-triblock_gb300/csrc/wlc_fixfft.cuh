@@ -17,7 +17,7 @@
 // additions between are exact to 2^-56 of the line's largest value, so the
 // error against 64-bit arithmetic is below that of FP64 butterflies.
 // Measured at 64^3, L = 10 (M = 121), launches timed one by one: pass A 1.42 ->
-// 0.65 ms, pass C 1.23 -> 0.37 ms, the two z-FFTs of pass B 0.6 ms less; one
+// 0.65 ms, pass C 1.23 -> 0.37 ms (0.53 and 0.34 with launch shapes by size), the two z-FFTs of pass B 0.6 ms less; one
 // step's error against 80-bit arithmetic 5.3e-16 -> 4.5e-16 of the result's
 // norm (1.50e-15 -> 1.45e-15 at the worst point).
 // Not-a-number and infinite inputs turn all outputs of their line into NaN;
