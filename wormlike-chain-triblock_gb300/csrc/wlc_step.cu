@@ -292,22 +292,25 @@ template <int N, int V = 0> __global__ void __launch_bounds__(512) ifft_xy(StepA
 // 64^3, L = 10: pass A 171 -> 147 us, pass C 109 -> 89 us; 128^3, L = 12: 2.65 ->
 // 2.42 and 1.70 -> 1.23 ms; 24^3, L = 8: 14.0 -> 11.1 and 12.2 -> 9.7 us.
 
-// x lines.  Pass A: in place, element (n, j) and output n + R j at slot n S + j,
-// R = N2, so that 16-byte vectors of a row stay together (J >= 8).  Pass C:
-// slot (j, k) at j S + k, R = N1, so that neighbouring lanes write >= 4
-// neighbours of a row.  S odd: neighbouring lanes on distinct banks.
+// x lines: J transforms of length R over elements n J + j, then R of length J,
+// the first radix first as along y and z, whichever pass it is (the order of
+// the additions, and with it every bit of an FP32 result, depends on it).
+// Pass A: in place, element (n, j) and output n + R j at slot n S + j.  J a
+// multiple of 4: S odd, lanes j-fastest (the four elements of a 16-byte vector
+// stay together).  Other J: natural order in rows of odd length, lanes
+// line-fastest.  Pass C: slot (j, k) at j S + k, S odd, so that neighbouring
+// lanes write >= 4 neighbours of a row.  Either way neighbouring lanes are on
+// distinct banks in both sub-passes.
 template <int N, bool FWD> struct XLine {
-    static constexpr int R = FWD ? Plan<N>::N2 : Plan<N>::N1, J = N / R;
-    static constexpr int S = (FWD ? J : R) | 1;
-    static constexpr int ROW = (FWD ? R : J) * S;
+    static constexpr int R = Plan<N>::N1, J = Plan<N>::N2;
+    static constexpr bool JFAST = J % 4 == 0;
+    static constexpr int S = !FWD ? R | 1 : JFAST ? J | 1 : J;
+    static constexpr int ROW = !FWD ? J * S : JFAST ? R * S : N + 1;
     __device__ __forceinline__ static int out_at(int k) { return (k % R) * S + k / R; }  // pass A, output k
 };
-template <int N> __host__ __device__ constexpr int xrow32(bool fwd) {
-    const int n1 = Plan<N>::N1, n2 = Plan<N>::N2;  // J of pass A and R of pass C are both N1
-    return fwd ? n2 * (n1 | 1) : n2 * (n1 | 1);
-}
+// row length that holds either pass's lines
 template <int N> __host__ __device__ constexpr int xrow32() {
-    return xrow32<N>(true) > xrow32<N>(false) ? xrow32<N>(true) : xrow32<N>(false);
+    return XLine<N, true>::ROW > XLine<N, false>::ROW ? XLine<N, true>::ROW : XLine<N, false>::ROW;
 }
 __host__ inline int xrow32_of(int N) {
     switch (N) {
@@ -346,7 +349,13 @@ __global__ void __launch_bounds__(512) rhs_fft_xy32(StepArgs<float> a0, const St
     constexpr int Z = XyShape<float, N, V>::Z, ZB = XyShape<float, N, V>::ZB;
     constexpr int NKX = N / 2 + 1, LS = NKX * Z, NR = N * N * N;
     using X = XLine<N, true>;
-    constexpr int R = X::R, J = X::J, YR = Plan<N>::N1, YJ = Plan<N>::N2;
+    constexpr int R = X::R, J = X::J;
+    static_assert(X::S == J || J % 4 == 0, "four consecutive x must lie on consecutive slots");
+    // item w of n x lines -> (line, n), the latter below n
+    auto item = [](int w, int n) {
+        if constexpr (X::JFAST) return int2{w / n, w % n};
+        return int2{w % (ZB * (N / 2)), w / (ZB * (N / 2))};
+    };
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2* tw = reinterpret_cast<float2*>(smem_raw);
     float2* zb = tw + N;                             // [ZB][N/2] packed row pairs, X::ROW each
@@ -374,48 +383,49 @@ __global__ void __launch_bounds__(512) rhs_fft_xy32(StepArgs<float> a0, const St
             }
         }
         __syncthreads();
-        if constexpr (R > 1) {
-            for (int w = threadIdx.x; w < ZB * (N / 2) * J; w += blockDim.x) {
-                const int j = w % J;
-                float2* row = zb + (size_t)(w / J) * X::ROW + j;
-                float2 v[R];
+        for (int w = threadIdx.x; w < ZB * (N / 2) * J; w += blockDim.x) {
+            const int2 t = item(w, J);
+            float2* row = zb + (size_t)t.x * X::ROW + t.y;
+            float2 v[R];
 #pragma unroll
-                for (int n = 0; n < R; ++n) v[n] = row[n * X::S];
-                Dft<R>::template run<-1>(v);
-                twiddles<R, -1>(v, j, tw);
+            for (int n = 0; n < R; ++n) v[n] = row[n * X::S];
+            Dft<R>::template run<-1>(v);
+            twiddles<R, -1>(v, t.y, tw);
 #pragma unroll
-                for (int n = 0; n < R; ++n) row[n * X::S] = v[n];
+            for (int n = 0; n < R; ++n) row[n * X::S] = v[n];
+        }
+        __syncthreads();
+        if constexpr (J > 1) {
+            for (int w = threadIdx.x; w < ZB * (N / 2) * R; w += blockDim.x) {
+                const int2 t = item(w, R);
+                float2* row = zb + (size_t)t.x * X::ROW + t.y * X::S;
+                float2 v[J];
+#pragma unroll
+                for (int j = 0; j < J; ++j) v[j] = row[j];
+                Dft<J>::template run<-1>(v);
+#pragma unroll
+                for (int j = 0; j < J; ++j) row[j] = v[j];
             }
             __syncthreads();
         }
-        for (int w = threadIdx.x; w < ZB * (N / 2) * R; w += blockDim.x) {
-            float2* row = zb + (size_t)(w / R) * X::ROW + (w % R) * X::S;
-            float2 v[J];
-#pragma unroll
-            for (int j = 0; j < J; ++j) v[j] = row[j];
-            Dft<J>::template run<-1>(v);
-#pragma unroll
-            for (int j = 0; j < J; ++j) row[j] = v[j];
-        }
-        __syncthreads();
         // first y sub-pass on the half spectra of rows (2p, 2p+1): lines (kx, plane)
-        for (LineWalk it(NKX * ZB); it.j < YJ; it.next()) {
+        for (LineWalk it(NKX * ZB); it.j < J; it.next()) {
             const int q = it.b % ZB, kx = it.b / ZB;
             const float2* zk = zb + (size_t)q * (N / 2) * X::ROW + X::out_at(kx);
             const float2* zm = zb + (size_t)q * (N / 2) * X::ROW + X::out_at((N - kx) % N);
-            float2 v[YR];
+            float2 v[R];
 #pragma unroll
-            for (int n = 0; n < YR; ++n) {
-                const int y = n * YJ + it.j;
+            for (int n = 0; n < R; ++n) {
+                const int y = n * J + it.j;
                 const float2 c = zk[(y >> 1) * X::ROW], d = zm[(y >> 1) * X::ROW];
                 v[n] = (y & 1) ? make_float2(0.5f * (c.y + d.y), 0.5f * (d.x - c.x))
                                : make_float2(0.5f * (c.x + d.x), 0.5f * (c.y - d.y));
             }
-            Dft<YR>::template run<-1>(v);
-            twiddles<YR, -1>(v, it.j, tw);
-            float2* o = out + (size_t)it.j * YR * LS + kx * Z + zz0 + q;
+            Dft<R>::template run<-1>(v);
+            twiddles<R, -1>(v, it.j, tw);
+            float2* o = out + (size_t)it.j * R * LS + kx * Z + zz0 + q;
 #pragma unroll
-            for (int k = 0; k < YR; ++k) o[k * LS] = v[k];
+            for (int k = 0; k < R; ++k) o[k * LS] = v[k];
         }
         __syncthreads();
     }
