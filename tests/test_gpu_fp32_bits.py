@@ -20,6 +20,7 @@ pytestmark = pytest.mark.gpu
 DIGESTS = {
     8: ["6983d1afb2863569", "f17f485fb1aa8a98"],
     12: ["df2537d1c7e6477d", "104fd0d01333e943"],
+    16: ["3e197515ce16a1bb", "0b33d9631f6e82f4"],
     24: ["613d23efbc745d52", "8f52e8267afb6fa9"],
     32: ["c9de756a5f9300f1", "1c46d53c925c2d1c"],
     40: ["6376c446077907da", "09bfd041b95864ab"],

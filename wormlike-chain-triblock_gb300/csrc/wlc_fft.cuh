@@ -174,10 +174,13 @@ template <> struct Dft<6> : DftCT<2, 3> {};
 template <> struct Dft<16> : DftCT<4, 4> {};
 
 // ------------------------------------------------------------ line plans
-// (16 as 4 x 4: one 16-point transform a thread left most of a small grid's
-// threads idle and each fetched its straight-line code cold; FP64 16^3, L = 2:
-// pass A 12.8 -> 9.1, B 39 -> 29, C 12.5 -> 8.5 us, FP32 within 3 % either way)
-template <int N> struct Plan;
+// (16 as 4 x 4 in the FP64 form: one 16-point transform a thread left most of a
+// small grid's threads idle and each fetched its straight-line code cold; 16^3,
+// L = 2: pass A 12.8 -> 9.1, B 39 -> 29, C 12.5 -> 8.5 us.  The FP32 form, where
+// it made no difference of more than 3 % either way, keeps the one transform and
+// with it the bits of its results.)
+template <int N, typename T = double> struct Plan : Plan<N> {};
+template <> struct Plan<16, float> { static constexpr int N1 = 16, N2 = 1; };
 template <> struct Plan<4> { static constexpr int N1 = 4, N2 = 1; };
 template <> struct Plan<6> { static constexpr int N1 = 6, N2 = 1; };
 template <> struct Plan<8> { static constexpr int N1 = 8, N2 = 1; };
@@ -192,13 +195,13 @@ template <> struct Plan<96> { static constexpr int N1 = 16, N2 = 6; };
 template <> struct Plan<128> { static constexpr int N1 = 16, N2 = 8; };
 
 // position of frequency (or output) index k after fft_nat2perm
-template <int N> __device__ __forceinline__ int perm_pos(int k) {
-    constexpr int N1 = Plan<N>::N1, N2 = Plan<N>::N2;
+template <int N, typename T = double> __device__ __forceinline__ int perm_pos(int k) {
+    constexpr int N1 = Plan<N, T>::N1, N2 = Plan<N, T>::N2;
     return (k % N1) * N2 + k / N1;
 }
 // index held at position p after fft_nat2perm
-template <int N> __device__ __forceinline__ int perm_index(int p) {
-    constexpr int N1 = Plan<N>::N1, N2 = Plan<N>::N2;
+template <int N, typename T = double> __device__ __forceinline__ int perm_index(int p) {
+    constexpr int N1 = Plan<N, T>::N1, N2 = Plan<N, T>::N2;
     return (p / N2) + N1 * (p % N2);
 }
 
@@ -232,7 +235,8 @@ struct LineWalk {
 // Batched in-place line FFTs: line b, element e at data[b*lstride + e*estride].
 template <int N, int DIR, typename C>
 __device__ __forceinline__ void fft_nat2perm(C* data, int nlines, int estride, int lstride, const C* tw) {
-    constexpr int N1 = Plan<N>::N1, N2 = Plan<N>::N2;
+    using P = Plan<N, decltype(C::x)>;
+    constexpr int N1 = P::N1, N2 = P::N2;
     if constexpr (N2 == 1) {
         for (int w = threadIdx.x; w < nlines; w += blockDim.x) {
             C* ln = data + (size_t)w * lstride;
@@ -276,7 +280,8 @@ __device__ __forceinline__ void fft_nat2perm(C* data, int nlines, int estride, i
 
 template <int N, int DIR, typename C>
 __device__ __forceinline__ void fft_perm2nat(C* data, int nlines, int estride, int lstride, const C* tw) {
-    constexpr int N1 = Plan<N>::N1, N2 = Plan<N>::N2;
+    using P = Plan<N, decltype(C::x)>;
+    constexpr int N1 = P::N1, N2 = P::N2;
     if constexpr (N2 == 1) {
         fft_nat2perm<N, DIR>(data, nlines, estride, lstride, tw);
     } else {

@@ -446,7 +446,7 @@ __global__ void __maxnreg__(sizeof(T) == 4 ? 80 : 128)
     const int p = threadIdx.x % N;
     const unsigned lmask = split.l[lpart], mmask = split.m[threadIdx.x / N];
     const T c0 = (T)a.c0, dcoef = (T)a.dcoef;
-    const int iz = fold_n(perm_index<N>(p), N), izr = fold_n(perm_index<N>(w / 2), N);
+    const int iz = fold_n(perm_index<N, T>(p), N), izr = fold_n(perm_index<N, T>(w / 2), N);
     const double kz = iz * a.kf[2];
     // angle of k to z and sigma ds |k|: in FP64 for FP64 propagators, in FP32
     // for FP32 ones (every thread runs this, and the FP64 pipe is a small

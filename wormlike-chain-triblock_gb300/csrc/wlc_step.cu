@@ -302,7 +302,7 @@ template <int N, int V = 0> __global__ void __launch_bounds__(512) ifft_xy(StepA
 // lanes write >= 4 neighbours of a row.  Either way neighbouring lanes are on
 // distinct banks in both sub-passes.
 template <int N, bool FWD> struct XLine {
-    static constexpr int R = Plan<N>::N1, J = Plan<N>::N2;
+    static constexpr int R = Plan<N, float>::N1, J = Plan<N, float>::N2;
     static constexpr bool JFAST = J % 4 == 0;
     static constexpr int S = !FWD ? R | 1 : JFAST ? J | 1 : J;
     static constexpr int ROW = !FWD ? J * S : JFAST ? R * S : N + 1;
@@ -332,7 +332,7 @@ template <int R, int DIR> __device__ __forceinline__ void twiddles(float2* v, in
 
 // second sub-pass of the y lines in place, f(line, ky, value) for every output
 template <int N, int DIR, int Z, typename F> __device__ __forceinline__ void y_second(float2* out, F&& f) {
-    constexpr int NKX = N / 2 + 1, LS = NKX * Z, R = Plan<N>::N1, J = Plan<N>::N2;
+    constexpr int NKX = N / 2 + 1, LS = NKX * Z, R = Plan<N, float>::N1, J = Plan<N, float>::N2;
     for (LineWalk it(LS); it.j < R; it.next()) {
         float2 v[J];
 #pragma unroll
@@ -466,8 +466,8 @@ __global__ void __launch_bounds__(512) ifft_xy32(StepArgs<float> a0, const StepA
         for (int w = threadIdx.x; w < ZB * (N / 2) * J; w += blockDim.x) {
             // plane fastest across the lanes, then j: neighbours in out
             const int q = w % ZB, j = w / ZB % J, p = w / (ZB * J), b = q * (N / 2) + p;
-            const float2* ra = out + (size_t)perm_pos<N>(2 * p) * LS + zz0 + q;
-            const float2* rb = out + (size_t)perm_pos<N>(2 * p + 1) * LS + zz0 + q;
+            const float2* ra = out + (size_t)perm_pos<N, float>(2 * p) * LS + zz0 + q;
+            const float2* rb = out + (size_t)perm_pos<N, float>(2 * p + 1) * LS + zz0 + q;
             float2 v[R];
 #pragma unroll
             for (int n = 0; n < R; ++n) v[n] = hermitian_pair<N>(ra, rb, n * J + j, Z);
