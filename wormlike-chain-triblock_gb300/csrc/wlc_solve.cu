@@ -176,15 +176,18 @@ __device__ __noinline__ void x_fx(long long* v, int vs, int l, int tr) {
     }
 }
 
-// the pair (x, y) rotated by an angle with cos, sin f (sgn < 0: by minus it)
+// the pair (x, y) rotated by an angle with cos, sin f (sgn < 0: by minus it).
+// The sign goes to the 64-bit numbers, never to the halves of the factor: a low
+// half of -2^31 has no negative in 32 bits (about one random box in a thousand
+// has such a sine, which then was off by 2^-30).
 __device__ __forceinline__ void dz_pair_fx(long long& x, long long& y, const fxw& f, int sgn) {
-    const fxh c = f.x, s = {sgn > 0 ? f.y.h : -f.y.h, sgn > 0 ? f.y.l : -f.y.l}, ns = {-s.h, -s.l};
     const fxh a = halves(x), b = halves(y);
+    const fxh sa = sgn > 0 ? a : halves(-x), sb = sgn > 0 ? halves(-y) : b;
     FixAcc u, w;
-    u.mad(c, a);
-    u.mad(ns, b);
-    w.mad(s, a);
-    w.mad(c, b);
+    u.mad(f.x, a);
+    u.mad(f.y, sb);
+    w.mad(f.y, sa);
+    w.mad(f.x, b);
     x = u.done();
     y = w.done();
 }
