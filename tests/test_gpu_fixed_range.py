@@ -29,3 +29,49 @@ def test_factor_whose_low_half_has_no_negative(L):
     assert np.abs(g.mde_one_step(4, pr) - ref).max() < 1e-14 * np.abs(ref).max()
     o.close()
     g.close()
+
+
+def _one_step(n, L, pr_of, lit=wlc.WLC_LIT_REAL4):
+    g = wlc.Instance(n, L, 10, (4, 2, 4), 1.2 / n, 1.3, (0.5, 0.6, 0.7), (15.0,) * 3, literals=lit)
+    rng = np.random.default_rng(700 + n)
+    q = g.mde_one_step(4, pr_of(rng.standard_normal((g.nr, g.M)) + 1.0))
+    g.close()
+    return q
+
+
+EDGES = [8, 12, 16, 24, 32, 40, 48, 64, 96]
+
+
+@pytest.mark.parametrize("n", EDGES)
+def test_overflow_of_the_literal_correction_is_not_finite(n):
+    """Real-4 literals: the first-order correction (from L = 2 on; the couplings
+    of L = 1 need none) runs in single precision.
+    Where a wavevector's coefficients leave its range (1e39 a point: beyond
+    3.4e38 at every wavevector) its sums are infinities and NaNs, and no
+    finite number may come out of the lines that they reach.  Well inside the
+    range the result is a number."""
+    assert np.isfinite(_one_step(n, 2, lambda pr: pr * 1e28)).all()
+    assert not np.isfinite(_one_step(n, 2, lambda pr: pr * 1e39)).any()
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("n", EDGES)
+def test_non_finite_input_with_the_correction(n, bad):
+    def put(pr):
+        pr[len(pr) // 2 + 3, 0] = bad
+        return pr
+    assert np.isnan(_one_step(n, 2, put)[:, 0]).all()
+
+
+def test_diverged_field_is_reported():
+    """Propagators that leave the correction's range end in WLC_E_NONFINITE, not in densities."""
+    n = 16
+    g = wlc.Instance(n, 2, 10, (4, 2, 4), 1.2 / n, 1.3, (0.5, 0.6, 0.7), (15.0,) * 3)
+    g.set_fields(np.random.default_rng(1).normal(-1e6, 1e5, size=(3, g.nr)))
+    g.MDE_q()
+    g.MDE_qstar()
+    assert np.abs(g.get_q(1, 5)).max() > 1e20
+    with pytest.raises(wlc.WlcError) as e:
+        g.density()
+    assert e.value.code == -5
+    g.close()

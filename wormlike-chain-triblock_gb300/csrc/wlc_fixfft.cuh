@@ -20,8 +20,8 @@
 // 0.65 ms, pass C 1.23 -> 0.37 ms (0.53 and 0.34 with launch shapes by size), the two z-FFTs of pass B 0.6 ms less; one
 // step's error against 80-bit arithmetic 5.3e-16 -> 4.5e-16 of the result's
 // norm (1.50e-15 -> 1.45e-15 at the worst point).
-// Not-a-number and infinite inputs turn all outputs of their line into NaN;
-// inputs below 2^-895 count as zero relative to 2^-895.
+// Not-a-number and infinite inputs, and a correction in floats that has
+// overflowed, turn all outputs of their line into NaN; inputs below 2^-895 count as zero relative to 2^-895.
 #pragma once
 #include <cstdint>
 
@@ -197,12 +197,15 @@ template <int N> __host__ __device__ constexpr int fx_exps(int nlines) {
 }
 
 // a float as a fixed-point number under exponent E >= fexp(f); subnormals count
-// as zero
-__device__ __forceinline__ int fexp(float f) { return ((__float_as_int(f) >> 23) & 0xff) + (1023 - 127); }
+// as zero.  fexp of an infinity or not-a-number: kExpBad
+__device__ __forceinline__ int fexp(float f) {
+    const int e = (__float_as_int(f) >> 23) & 0xff;
+    return e == 255 ? kExpBad : e + (1023 - 127);
+}
 __device__ __forceinline__ fx f2fx(float f, int E) {
     const int u = __float_as_int(f), e = (u >> 23) & 0xff;
     const long long m = (long long)((u & 0x7fffff) | 0x800000) << (kTop - 22);
-    const long long v = e == 0 ? 0 : round_shift(m, E - fexp(f) + 1);
+    const long long v = e == 0 ? 0 : round_shift(m, E - (e + 1023 - 127) + 1);
     return mkfx(u < 0 ? -v : v);
 }
 
