@@ -75,3 +75,15 @@ def test_diverged_field_is_reported():
         g.density()
     assert e.value.code == -5
     g.close()
+
+
+@pytest.mark.parametrize("n", EDGES)
+def test_small_numbers_with_the_correction(n):
+    """The step is linear: inputs scaled by 2^k give outputs scaled by 2^k.  With
+    real-4 literals as long as the correction, a few 2^-24 of the result, stays
+    in single precision's range (k = -60: to the rounding of the step, 1e-14);
+    below, to the size of the correction that is lost, under 1e-6."""
+    q = _one_step(n, 2, lambda pr: pr)
+    for k, tol in ((-60, 1e-14), (-110, 1e-6), (-140, 1e-6), (-170, 1e-6), (-300, 1e-6), (-800, 1e-6)):
+        s = np.ldexp(_one_step(n, 2, lambda pr: np.ldexp(pr, k)), -k)
+        assert np.abs(s - q).max() <= tol * np.abs(q).max()

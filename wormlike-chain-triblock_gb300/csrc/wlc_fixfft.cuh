@@ -128,13 +128,15 @@ static __device__ __noinline__ double fx2d_rare(long long v, int E) {
     return E >= kExpBad / 2 ? __longlong_as_double(0x7ff8000000000000LL) : ldexp((double)v, E - 1023 - kTop);
 }
 // d as a float, round to nearest even, on the integer ALUs (the conversion
-// instruction runs on the FP64 pipe); below 2^-126 zero
+// instruction runs on the FP64 pipe; only subnormal floats go there)
+static __device__ __noinline__ float d2f_rare(double d) { return __double2float_rn(d); }
 __device__ __forceinline__ float d2f(double d) {
     const long long b = __double_as_longlong(d);
     const long long r = b + 0x0fffffff + ((b >> 29) & 1);
     const int e = (int)((r >> 52) & 0x7ff) - (1023 - 127);
     const unsigned m = (unsigned)(r >> 29) & 0x7fffffu, sg = (unsigned)(b >> 32) & 0x80000000u;
-    return __uint_as_float(e <= 0 ? sg : e >= 255 ? sg | 0x7f800000u | ((b << 1) > (0x7ffLL << 53) ? 1u : 0u)
+    if (e <= 0 && (unsigned long long)b << 1 != 0) return d2f_rare(d);
+    return __uint_as_float(e <= 0 ? sg : e >= 255 ? sg | 0x7f800000u | ((unsigned long long)b << 1 > 0x7ffull << 53 ? 1u : 0u)
                                                   : sg | ((unsigned)e << 23) | m);
 }
 // v under exponent E as a double by the conversion instruction: fewer
@@ -196,16 +198,17 @@ template <int N> __host__ __device__ constexpr int fx_exps(int nlines) {
     return Plan<N>::N2 == 1 ? 0 : nlines * (Plan<N>::N1 > Plan<N>::N2 ? Plan<N>::N1 : Plan<N>::N2);
 }
 
-// a float as a fixed-point number under exponent E >= fexp(f); subnormals count
-// as zero.  fexp of an infinity or not-a-number: kExpBad
+// a float as a fixed-point number under exponent E >= fexp(f).  fexp of zero: 0
+// (a correction that vanishes must not raise its line's exponent); of an
+// infinity or not-a-number: kExpBad
 __device__ __forceinline__ int fexp(float f) {
-    const int e = (__float_as_int(f) >> 23) & 0xff;
-    return e == 255 ? kExpBad : e + (1023 - 127);
+    const int u = __float_as_int(f), e = (u >> 23) & 0xff;
+    return e == 255 ? kExpBad : u << 1 == 0 ? 0 : max(e, 1) + (1023 - 127);
 }
 __device__ __forceinline__ fx f2fx(float f, int E) {
     const int u = __float_as_int(f), e = (u >> 23) & 0xff;
-    const long long m = (long long)((u & 0x7fffff) | 0x800000) << (kTop - 22);
-    const long long v = e == 0 ? 0 : round_shift(m, E - (e + 1023 - 127) + 1);
+    const long long m = (long long)((u & 0x7fffff) | (e ? 0x800000 : 0)) << (kTop - 22);
+    const long long v = round_shift(m, E - (max(e, 1) + 1023 - 127) + 1);
     return mkfx(u < 0 ? -v : v);
 }
 
