@@ -87,3 +87,29 @@ def test_small_numbers_with_the_correction(n):
     for k, tol in ((-60, 1e-14), (-110, 1e-6), (-140, 1e-6), (-170, 1e-6), (-300, 1e-6), (-800, 1e-6)):
         s = np.ldexp(_one_step(n, 2, lambda pr: np.ldexp(pr, k)), -k)
         assert np.abs(s - q).max() <= tol * np.abs(q).max()
+
+
+@pytest.mark.parametrize("n", EDGES)
+def test_tiny_numbers(n):
+    """Down to where doubles themselves lose bits, scaling the input by 2^k scales
+    the output: 2^-930 and 2^-990 times numbers over twelve decades, against
+    the unscaled step to its rounding (1e-14 of the largest output; the
+    smallest subnormal is 2^-84 of the largest number even at k = -990).
+    Tiny next to ordinary coefficients, and an input of zeros."""
+    def spread(pr):
+        return pr * 10.0 ** np.linspace(-12, 0, pr.shape[1])
+
+    q = _one_step(n, 2, spread, wlc.WLC_LIT_REAL8)
+    for k in (-930, -990):
+        s = np.ldexp(_one_step(n, 2, lambda pr: np.ldexp(spread(pr), k), wlc.WLC_LIT_REAL8), -k)
+        assert np.abs(s - q).max() <= 1e-14 * np.abs(q).max()
+
+    def one_tiny(pr):
+        pr[:, 0] = np.ldexp(pr[:, 0], -1000)
+        return pr
+
+    # as without it
+    a, b = _one_step(n, 2, one_tiny), _one_step(n, 2, lambda pr: pr * (np.arange(pr.shape[1]) > 0))
+    assert np.abs(a - b).max() <= 1e-14 * np.abs(b).max()
+    for lit in (wlc.WLC_LIT_REAL4, wlc.WLC_LIT_REAL8):
+        assert not _one_step(n, 2, lambda pr: pr * 0.0, lit).any()

@@ -21,7 +21,10 @@
 // step's error against 80-bit arithmetic 5.3e-16 -> 4.5e-16 of the result's
 // norm (1.50e-15 -> 1.45e-15 at the worst point).
 // Not-a-number and infinite inputs, and a correction in floats that has
-// overflowed, turn all outputs of their line into NaN; inputs below 2^-895 count as zero relative to 2^-895.
+// overflowed, turn all outputs of their line into NaN.  Elements that are all
+// below 2^-895 are multiplied by 2^512 first (lift_tiny), down to the smallest
+// subnormal; results below 2^-920 or above 2^977 are rounded by the library's
+// ldexp.
 #pragma once
 #include <cstdint>
 
@@ -30,8 +33,10 @@
 namespace wlc {
 
 constexpr int kTop = 56;       // bit of the largest component after normalisation
-constexpr int kExpMin = 128;   // smallest shared (biased) exponent
-constexpr int kExpBad = 20000; // exponent of a line with non-finite input
+constexpr int kExpLow = 128;    // biased exponent below which inputs are lifted (an exponent field of 0 needs 64 below it)
+constexpr int kLift = 512;
+constexpr int kExpMin = -1500;  // exponent of zeros: below that of every other number
+constexpr int kExpBad = 20000;  // exponent of a line with non-finite input
 
 // a fixed-point number; as a constant it holds value * 2^62
 struct fx {
@@ -124,8 +129,25 @@ template <int TOP = kTop> __device__ __forceinline__ fx d2fx(double d, int E) {
     const long long sg = (long long)(hi >> 31);
     return mkfx((v ^ sg) - sg);
 }
-static __device__ __noinline__ double fx2d_rare(long long v, int E) {
+// value of v under an exponent for which fx2d and fx2d_cvt do not hold
+__device__ __forceinline__ bool fx_rare(int E) { return (unsigned)(E - 100) >= 1900u; }
+static __device__ __noinline__ double fx2d_ldexp(long long v, int E) {
     return E >= kExpBad / 2 ? __longlong_as_double(0x7ff8000000000000LL) : ldexp((double)v, E - 1023 - kTop);
+}
+__device__ __forceinline__ double fx2d_rare(long long v, int E) { return v == 0 && E < 2000 ? 0.0 : fx2d_ldexp(v, E); }
+// the doubles v[j * step + c], j < n, c < width, times 2^kLift (exact); returns
+// the largest exponent field then, 0 if all are zero
+static __device__ __noinline__ int lift_tiny(double* v, int step, int n, int width) {
+    int E = 0;
+#pragma unroll 1
+    for (int j = 0; j < n; ++j)
+#pragma unroll 1
+        for (int c = 0; c < width; ++c) {
+            const double x = v[j * step + c] * 0x1p512;
+            v[j * step + c] = x;
+            E = max(E, dexp(x));
+        }
+    return E;
 }
 // d as a float, round to nearest even, on the integer ALUs (the conversion
 // instruction runs on the FP64 pipe; only subnormal floats go there)
@@ -161,7 +183,7 @@ __device__ __forceinline__ double fx2d(fx q, int E) {
 
 // E of R complex doubles
 template <int R> __device__ __forceinline__ int shared_exp(const double2* d) {
-    int E = kExpMin;
+    int E = 0;
 #pragma unroll
     for (int n = 0; n < R; ++n) E = max(E, max(dexp(d[n].x), dexp(d[n].y)));
     return E == 2047 ? kExpBad : E;
@@ -231,7 +253,7 @@ template <typename F> __device__ __forceinline__ FromFixed<F> from_fixed(F f) { 
 
 // the R elements base + n*step of line b into registers; returns the exponent
 template <int R, typename In>
-__device__ __forceinline__ int fx_load(const double2* ln, int estride, int b, int base, int step, const In& in, fxc* v) {
+__device__ __forceinline__ int fx_load(double2* ln, int estride, int b, int base, int step, const In& in, fxc* v) {
     if constexpr (In::dbl) {
         double2 d[R];
 #pragma unroll
@@ -246,6 +268,14 @@ __device__ __forceinline__ int fx_load(const double2* ln, int estride, int b, in
             }
             E = E < kExpBad ? E + 1 : E;  // room for the difference
         }
+        int lift = 0;
+        if (E < kExpLow) {  // tiny numbers or zeros (and no correction)
+            const int e = lift_tiny(reinterpret_cast<double*>(ln + base * estride), 2 * step * estride, R, 2);
+#pragma unroll
+            for (int n = 0; n < R; ++n) d[n] = ln[(base + n * step) * estride];
+            E = max(e + (In::less ? 1 : 0), kExpLow);
+            lift = e > 0 ? kLift : kExpLow - kExpMin;
+        }
 #pragma unroll
         for (int n = 0; n < R; ++n) {
             v[n].x = d2fx(d[n].x, E);
@@ -255,7 +285,7 @@ __device__ __forceinline__ int fx_load(const double2* ln, int estride, int b, in
                 v[n].y = v[n].y - f2fx(c[n].y, E);
             }
         }
-        return E;
+        return E - lift;
     } else {
         int e[R];
 #pragma unroll
@@ -270,7 +300,7 @@ __device__ __forceinline__ int fx_load(const double2* ln, int estride, int b, in
 template <int R, bool OUTD>
 __device__ __forceinline__ void fx_store(double2* ln, int estride, int base, int step, const fxc* v, int E) {
     if constexpr (OUTD) {
-        const bool rare = E >= 2000;
+        const bool rare = fx_rare(E);
 #pragma unroll
         for (int n = 0; n < R; ++n) {
             double2 d;

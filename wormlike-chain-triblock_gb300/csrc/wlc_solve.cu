@@ -203,9 +203,14 @@ __device__ __noinline__ void rot_all_fx(double* __restrict__ v0, int vs, int L, 
         double* const vd = v0 + l * l * vs;          // first element (m = -l)
         long long* const v = reinterpret_cast<long long*>(vd);
         const int mid = l * vs;                      // m = 0
-        int E = kExpMin;
+        int E = 0, lift = 0;
 #pragma unroll 4
         for (int j = 0; j < 2 * l + 1; ++j) E = max(E, (reinterpret_cast<const int*>(vd + j * vs)[1] >> 20) & 0x7ff);
+        if (E < kExpLow) {
+            E = lift_tiny(vd, vs, 2 * l + 1, 1);
+            if (E == 0) continue;  // zeros stay zeros
+            lift = kLift;
+        }
         if (E == 2047) E = kExpBad;
         v[mid] = d2fx<kRotTop>(vd[mid], E).v;
 #pragma unroll 2
@@ -225,8 +230,8 @@ __device__ __noinline__ void rot_all_fx(double* __restrict__ v0, int vs, int L, 
             v[py] = y;
         }
         x_fx(v, vs, l, 1);
-        const bool rare = E >= 2000;
-        E += kTop - kRotTop;
+        E += kTop - kRotTop - lift;
+        const bool rare = fx_rare(E);
         vd[mid] = rare ? fx2d_rare(v[mid], E) : fx2d_cvt(v[mid], E);
 #pragma unroll 2
         for (int m = 1; m <= l; ++m) {
