@@ -21,10 +21,9 @@
 // step's error against 80-bit arithmetic 5.3e-16 -> 4.5e-16 of the result's
 // norm (1.50e-15 -> 1.45e-15 at the worst point).
 // Not-a-number and infinite inputs, and a correction in floats that has
-// overflowed, turn all outputs of their line into NaN.  Elements that are all
-// below 2^-895 are multiplied by 2^512 first (lift_tiny), down to the smallest
-// subnormal; results below 2^-920 or above 2^977 are rounded by the library's
-// ldexp.
+// overflowed, turn all outputs of their line into NaN.  Numbers keep their
+// bits down to the smallest subnormal; results below 2^-920 or above 2^977 are
+// rounded by the library's ldexp.
 #pragma once
 #include <cstdint>
 
@@ -33,9 +32,9 @@
 namespace wlc {
 
 constexpr int kTop = 56;       // bit of the largest component after normalisation
-constexpr int kExpLow = 128;    // biased exponent below which inputs are lifted (an exponent field of 0 needs 64 below it)
+constexpr int kExpLow = 64;     // shared (biased) exponents below are tiny numbers: d2fx_low, lift_tiny
 constexpr int kLift = 512;
-constexpr int kExpMin = -1500;  // exponent of zeros: below that of every other number
+constexpr int kExpMin = -100;   // below every shared exponent
 constexpr int kExpBad = 20000;  // exponent of a line with non-finite input
 
 // a fixed-point number; as a constant it holds value * 2^62
@@ -119,7 +118,8 @@ __device__ __forceinline__ long long sar_s64(long long v, int s) {  // sign for 
 }
 // v / 2^s to the nearest, s >= 1 (halves up; 0 or so for s > 64)
 __device__ __forceinline__ long long round_shift(long long v, int s) { return (sar_s64(v, s - 1) + 1) >> 1; }
-// d as a fixed-point number under exponent E >= d's own (E's leading bit at TOP)
+// d as a fixed-point number under exponent E >= d's own (E's leading bit at
+// TOP), E >= kExpLow (a zero or subnormal d then counts as zero)
 template <int TOP = kTop> __device__ __forceinline__ fx d2fx(double d, int E) {
     const int hi = __double2hiint(d), lo = __double2loint(d);
     const int s = E - ((hi >> 20) & 0x7ff);
@@ -129,37 +129,44 @@ template <int TOP = kTop> __device__ __forceinline__ fx d2fx(double d, int E) {
     const long long sg = (long long)(hi >> 31);
     return mkfx((v ^ sg) - sg);
 }
+// the same under any E >= 1, for subnormal d as well
+__device__ __forceinline__ fx d2fx_low(double d, int E) {
+    const long long b = __double_as_longlong(d);
+    const int e = dexp(d);
+    const unsigned long long m = ((b & 0xfffffffffffffll) | (e ? 1ll << 52 : 0ll)) << (kTop - 51);
+    const long long v = (long long)((shr_u64(m, E - max(e, 1)) + 1) >> 1);
+    return mkfx(b < 0 ? -v : v);
+}
 // value of v under an exponent for which fx2d and fx2d_cvt do not hold
 __device__ __forceinline__ bool fx_rare(int E) { return (unsigned)(E - 100) >= 1900u; }
-static __device__ __noinline__ double fx2d_ldexp(long long v, int E) {
-    return E >= kExpBad / 2 ? __longlong_as_double(0x7ff8000000000000LL) : ldexp((double)v, E - 1023 - kTop);
+static __device__ __noinline__ double fx2d_rare(long long v, int E) {
+    if (E >= kExpBad / 2) return __longlong_as_double(0x7ff8000000000000LL);
+    return v == 0 ? 0.0 : ldexp((double)v, E - 1023 - kTop);
 }
-__device__ __forceinline__ double fx2d_rare(long long v, int E) { return v == 0 && E < 2000 ? 0.0 : fx2d_ldexp(v, E); }
-// the doubles v[j * step + c], j < n, c < width, times 2^kLift (exact); returns
-// the largest exponent field then, 0 if all are zero
-static __device__ __noinline__ int lift_tiny(double* v, int step, int n, int width) {
+// the doubles v[j * step], j < n, times 2^kLift (exact); returns the largest
+// exponent field then, 0 if all are zero
+static __device__ __noinline__ int lift_tiny(double* v, int step, int n) {
     int E = 0;
 #pragma unroll 1
-    for (int j = 0; j < n; ++j)
-#pragma unroll 1
-        for (int c = 0; c < width; ++c) {
-            const double x = v[j * step + c] * 0x1p512;
-            v[j * step + c] = x;
-            E = max(E, dexp(x));
-        }
+    for (int j = 0; j < n; ++j) {
+        const double x = v[j * step] * 0x1p512;
+        v[j * step] = x;
+        E = max(E, dexp(x));
+    }
     return E;
 }
 // d as a float, round to nearest even, on the integer ALUs (the conversion
-// instruction runs on the FP64 pipe; only subnormal floats go there)
-static __device__ __noinline__ float d2f_rare(double d) { return __double2float_rn(d); }
+// instruction runs on the FP64 pipe; only zeros and what becomes a subnormal
+// float go there)
 __device__ __forceinline__ float d2f(double d) {
     const long long b = __double_as_longlong(d);
     const long long r = b + 0x0fffffff + ((b >> 29) & 1);
     const int e = (int)((r >> 52) & 0x7ff) - (1023 - 127);
     const unsigned m = (unsigned)(r >> 29) & 0x7fffffu, sg = (unsigned)(b >> 32) & 0x80000000u;
-    if (e <= 0 && (unsigned long long)b << 1 != 0) return d2f_rare(d);
-    return __uint_as_float(e <= 0 ? sg : e >= 255 ? sg | 0x7f800000u | ((unsigned long long)b << 1 > 0x7ffull << 53 ? 1u : 0u)
-                                                  : sg | ((unsigned)e << 23) | m);
+    float f = __uint_as_float(e >= 255 ? sg | 0x7f800000u | ((unsigned long long)b << 1 > 0x7ffull << 53 ? 1u : 0u)
+                                       : sg | ((unsigned)e << 23) | m);
+    asm("{ .reg .pred p; setp.le.s32 p, %2, 0; @p cvt.rn.f32.f64 %0, %1; }" : "+f"(f) : "d"(d), "r"(e));
+    return f;
 }
 // v under exponent E as a double by the conversion instruction: fewer
 // instructions than fx2d, on the FP64 pipe (for loops whose other work is on
@@ -220,12 +227,11 @@ template <int N> __host__ __device__ constexpr int fx_exps(int nlines) {
     return Plan<N>::N2 == 1 ? 0 : nlines * (Plan<N>::N1 > Plan<N>::N2 ? Plan<N>::N1 : Plan<N>::N2);
 }
 
-// a float as a fixed-point number under exponent E >= fexp(f).  fexp of zero: 0
-// (a correction that vanishes must not raise its line's exponent); of an
-// infinity or not-a-number: kExpBad
-__device__ __forceinline__ int fexp(float f) {
-    const int u = __float_as_int(f), e = (u >> 23) & 0xff;
-    return e == 255 ? kExpBad : u << 1 == 0 ? 0 : max(e, 1) + (1023 - 127);
+// a float as a fixed-point number under exponent E >= fexp of the largest |f|'s
+// bits.  fexp of zero: 0 (a correction that vanishes must not raise its line's
+// exponent); of an infinity or not-a-number: kExpBad
+__device__ __forceinline__ int fexp(int u) {
+    return u >= 0x7f800000 ? kExpBad : u == 0 ? 0 : max(u >> 23, 1) + (1023 - 127);
 }
 __device__ __forceinline__ fx f2fx(float f, int E) {
     const int u = __float_as_int(f), e = (u >> 23) & 0xff;
@@ -253,7 +259,7 @@ template <typename F> __device__ __forceinline__ FromFixed<F> from_fixed(F f) { 
 
 // the R elements base + n*step of line b into registers; returns the exponent
 template <int R, typename In>
-__device__ __forceinline__ int fx_load(double2* ln, int estride, int b, int base, int step, const In& in, fxc* v) {
+__device__ __forceinline__ int fx_load(const double2* ln, int estride, int b, int base, int step, const In& in, fxc* v) {
     if constexpr (In::dbl) {
         double2 d[R];
 #pragma unroll
@@ -261,20 +267,23 @@ __device__ __forceinline__ int fx_load(double2* ln, int estride, int b, int base
         int E = shared_exp<R>(d);
         float2 c[In::less ? R : 1];
         if constexpr (In::less) {
+            int u = 0;
 #pragma unroll
             for (int n = 0; n < R; ++n) {
                 c[n] = in.c[b * in.stride + base + n * step];
-                E = max(E, max(fexp(c[n].x), fexp(c[n].y)));
+                u = max(u, max(__float_as_int(c[n].x) & 0x7fffffff, __float_as_int(c[n].y) & 0x7fffffff));
             }
+            E = max(E, fexp(u));
             E = E < kExpBad ? E + 1 : E;  // room for the difference
         }
-        int lift = 0;
         if (E < kExpLow) {  // tiny numbers or zeros (and no correction)
-            const int e = lift_tiny(reinterpret_cast<double*>(ln + base * estride), 2 * step * estride, R, 2);
+            E = max(E, 1);
 #pragma unroll
-            for (int n = 0; n < R; ++n) d[n] = ln[(base + n * step) * estride];
-            E = max(e + (In::less ? 1 : 0), kExpLow);
-            lift = e > 0 ? kLift : kExpLow - kExpMin;
+            for (int n = 0; n < R; ++n) {
+                v[n].x = d2fx_low(d[n].x, E);
+                v[n].y = d2fx_low(d[n].y, E);
+            }
+            return E;
         }
 #pragma unroll
         for (int n = 0; n < R; ++n) {
@@ -285,7 +294,7 @@ __device__ __forceinline__ int fx_load(double2* ln, int estride, int b, int base
                 v[n].y = v[n].y - f2fx(c[n].y, E);
             }
         }
-        return E - lift;
+        return E;
     } else {
         int e[R];
 #pragma unroll

@@ -207,7 +207,7 @@ __device__ __noinline__ void rot_all_fx(double* __restrict__ v0, int vs, int L, 
 #pragma unroll 4
         for (int j = 0; j < 2 * l + 1; ++j) E = max(E, (reinterpret_cast<const int*>(vd + j * vs)[1] >> 20) & 0x7ff);
         if (E < kExpLow) {
-            E = lift_tiny(vd, vs, 2 * l + 1, 1);
+            E = lift_tiny(vd, vs, 2 * l + 1);
             if (E == 0) continue;  // zeros stay zeros
             lift = kLift;
         }
