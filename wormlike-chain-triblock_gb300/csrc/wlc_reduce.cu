@@ -288,10 +288,23 @@ __global__ void __launch_bounds__(Pts<T>::THREADS)
 // a product and its error are exact in two floats and are added to a sum of
 // three floats by error-free additions (72 bits; the FP64 pipe has 1/64 of
 // the FP32 rate, and one multiply-add with its two conversions costs 192
-// clocks of a scheduler there against 22 here).
+// clocks of a scheduler there against 24 here).  That holds while the largest
+// product lies within 2^-90 .. 2^100: errors of smaller products, below 2^-149,
+// are then under 2^-59 of it and no sum overflows.  Otherwise (and for zeros
+// and not-a-numbers) holds() is false and dot_fp64 sums again in FP64.
 __device__ __forceinline__ float two_sum(float a, float b, float& err) {
     const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
     err = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+    return s;
+}
+// sum over the rows first, first + step, ... < M (through order, if given) of a c
+static __device__ __noinline__ double dot_fp64(const float* a, const float* c, const int16_t* order, int first, int step,
+                                               int M, int64_t nr) {
+    double s = 0.0;
+    for (int row = first; row < M; row += step) {
+        const int64_t o = (order ? order[row] : row) * nr;
+        s = fma((double)a[o], (double)c[o], s);
+    }
     return s;
 }
 template <typename T, int P> struct Dots;
@@ -299,13 +312,11 @@ template <int P> struct Dots<double, P> {
     static constexpr int W = 1;  // words per point
     double s[P] = {};
     __device__ __forceinline__ void add(int u, double a, double b) { s[u] = fma(a, b, s[u]); }
-    __device__ __forceinline__ void put(int u, double* w, int) const { w[0] = s[u]; }
-    __device__ __forceinline__ void merge(int u, const double* w, int) { s[u] += w[0]; }
     __device__ __forceinline__ double get(int u) const { return s[u]; }
 };
 template <int P> struct Dots<float, P> {
     static constexpr int W = 3;
-    float s[P] = {}, c[P] = {}, d[P] = {};
+    float s[P] = {}, c[P] = {}, d[P] = {}, top[P] = {};  // top: largest product
     __device__ __forceinline__ void add3(int u, float p, float e, float f) {
         float t1, t2, t3;
         s[u] = two_sum(s[u], p, t1);
@@ -315,19 +326,11 @@ template <int P> struct Dots<float, P> {
     }
     __device__ __forceinline__ void add(int u, float a, float b) {
         const float p = __fmul_rn(a, b);
+        top[u] = fmaxf(top[u], fabsf(p));
         add3(u, p, __fmaf_rn(a, b, -p), 0.0f);
     }
-    __device__ __forceinline__ void put(int u, float* w, int st) const {
-        w[0] = s[u];
-        w[st] = c[u];
-        w[2 * st] = d[u];
-    }
-    __device__ __forceinline__ void merge(int u, const float* w, int st) { add3(u, w[0], w[st], w[2 * st]); }
-    // an overflow leaves a not-a-number in the error terms: the sum itself says which
-    __device__ __forceinline__ double get(int u) const {
-        const double e = (double)c[u] + (double)d[u];
-        return isfinite(s[u]) && isfinite(e) ? (double)s[u] + e : (double)s[u];
-    }
+    __device__ __forceinline__ bool holds(int u) const { return top[u] >= 0x1p-90f && top[u] <= 0x1p100f && s[u] == s[u]; }
+    __device__ __forceinline__ double get(int u) const { return (double)s[u] + ((double)c[u] + (double)d[u]); }
 };
 
 // raw[b][r] = sum_i S1_{s in block b}(q_i q*_i); junc[j][r] = sum_i q_i q*_i at
@@ -384,7 +387,11 @@ __global__ void __launch_bounds__(256)
         }
         double v[P];
 #pragma unroll
-        for (int u = 0; u < P; ++u) v[u] = dot.get(u);
+        for (int u = 0; u < P; ++u) {
+            v[u] = dot.get(u);
+            if constexpr (sizeof(T) == 4)
+                if (in && !dot.holds(u)) v[u] = dot_fp64(qf + s * sl + r + u, qb + s * sl + r + u, nullptr, g, G, d.M, nr);
+        }
         for (int b = 0; b < 3; ++b) {
             const int j = s - d.nstart[b], n = d.ns[b];
             if (n <= 0 || j < 0 || j > n) continue;
@@ -475,7 +482,20 @@ __device__ __forceinline__ void slice_sums(const T* __restrict__ a, const T* __r
     T* red = tile + (size_t)g * (W + 5) * TILE + k;
 #pragma unroll
     for (int u = 0; u < P; ++u) {
-        dot.put(u, red + u, TILE);
+        if constexpr (sizeof(T) == 8) {
+            red[u] = dot.get(u);
+        } else {  // the three words of the sum, or the two of an FP64 sum and a not-a-number
+            red[u] = dot.s[u];
+            red[TILE + u] = dot.c[u];
+            red[2 * TILE + u] = dot.d[u];
+            if (!dot.holds(u)) {
+                const int64_t o = r0 + k + u;
+                const double v = dot_fp64(a + o, c + o, lists ? lists->order : nullptr, g, kGroups, M, nr);
+                red[u] = __int_as_float(__double2hiint(v));
+                red[TILE + u] = __int_as_float(__double2loint(v));
+                red[2 * TILE + u] = __int_as_float(0x7fc00000);
+            }
+        }
         if (lists)
 #pragma unroll
             for (int t = 0; t < 5; ++t) red[(W + t) * TILE + u] = f[t][u];
@@ -485,9 +505,21 @@ __device__ __forceinline__ void slice_sums(const T* __restrict__ a, const T* __r
 // the tile's point k: the dot product, and tensor component t
 template <typename T> __device__ __forceinline__ double slice_dot(const T* red, int k) {
     constexpr int TILE = PointTile<T>::value, W = Dots<T, 1>::W;
+    double x = 0.0;
     Dots<T, 1> dot;
-    for (int g = 0; g < kGroups; ++g) dot.merge(0, red + (size_t)g * (W + 5) * TILE + k, TILE);
-    return dot.get(0);
+    for (int g = 0; g < kGroups; ++g) {
+        const T* w = red + (size_t)g * (W + 5) * TILE + k;
+        if constexpr (sizeof(T) == 8) {
+            x += w[0];
+        } else {
+            const float d = w[2 * TILE];
+            if (d == d)
+                dot.add3(0, w[0], w[TILE], d);
+            else
+                x += __hiloint2double(__float_as_int(w[0]), __float_as_int(w[TILE]));
+        }
+    }
+    return dot.get(0) + x;
 }
 template <typename T> __device__ __forceinline__ double slice_form(const T* red, int t, int k) {
     constexpr int TILE = PointTile<T>::value, W = Dots<T, 1>::W;
