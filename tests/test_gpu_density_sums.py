@@ -82,3 +82,29 @@ def test_fp32_densities_of_small_propagators(n, store):
     assert (np.abs(d["junction"][[0, 2]] - junc) <= 14 * 2.0 ** -52 * junc).all()
     g.close()
     ref.close()
+
+
+def test_fp64_sum_is_no_single_chain():
+    """121 coefficients whose products are 1 and then 1.5 * 2^-53 each: added one
+    after the other every addition rounds up by half a unit of 2^-53, 60 in
+    all.  Sums of every fourth product round at most 31 times, join in 2
+    additions, and five slices add up and scale in 9: 42 units.  Relative to
+    the points whose products but the first are zero and whose sums are exact."""
+    n, L = 64, 10
+    g = wlc.Instance(n, L, NMAX, NS, 1.2 / n, 1.3, (0.5,) * 3, (15.0,) * 3)
+    g.set_fields(np.zeros((3, g.nr)))
+    g.MDE_q()
+    g.MDE_qstar()
+    q = np.zeros((g.nr, g.M))
+    q[:, 0] = 1.0
+    p = q.copy()
+    q[::2, 1:] = 1.0
+    p[::2, 1:] = 1.5 * 2.0 ** -53
+    for s in range(NMAX + 1):
+        g.set_q(1, s, q)
+        g.set_q(-1, s, p)
+    phi = g.density(want_junction=False)["phi"][:2]
+    g.close()
+    exact = 120 * 1.5  # units of 2^-53 above 1
+    off = (phi[:, ::2] - phi[:, 1::2]) / phi[:, 1::2] * 2.0 ** 53 - exact
+    assert np.abs(off).max() <= 42

@@ -307,14 +307,19 @@ static __device__ __noinline__ double dot_fp64(const float* a, const float* c, c
     }
     return s;
 }
-template <typename T, int P> struct Dots;
-template <int P> struct Dots<double, P> {
+// FP64 slices: K sums of every K-th product (add's k), so that a long row of
+// coefficients is not one chain of roundings
+template <typename T, int P, int K = 1> struct Dots;
+template <int P, int K> struct Dots<double, P, K> {
     static constexpr int W = 1;  // words per point
-    double s[P] = {};
-    __device__ __forceinline__ void add(int u, double a, double b) { s[u] = fma(a, b, s[u]); }
-    __device__ __forceinline__ double get(int u) const { return s[u]; }
+    double s[K][P] = {};
+    __device__ __forceinline__ void add(int u, double a, double b, int k = 0) { s[k][u] = fma(a, b, s[k][u]); }
+    __device__ __forceinline__ double get(int u) const {
+        if constexpr (K == 4) return (s[0][u] + s[1][u]) + (s[2][u] + s[3][u]);
+        return s[0][u];
+    }
 };
-template <int P> struct Dots<float, P> {
+template <int P, int K> struct Dots<float, P, K> {
     static constexpr int W = 3;
     float s[P] = {}, c[P] = {}, d[P] = {}, top[P] = {};  // top: largest product
     __device__ __forceinline__ void add3(int u, float p, float e, float f) {
@@ -324,7 +329,7 @@ template <int P> struct Dots<float, P> {
         c[u] = two_sum(c[u], e, t3);
         d[u] = __fadd_rn(d[u], __fadd_rn(__fadd_rn(t2, t3), f));
     }
-    __device__ __forceinline__ void add(int u, float a, float b) {
+    __device__ __forceinline__ void add(int u, float a, float b, int = 0) {
         const float p = __fmul_rn(a, b);
         top[u] = fmaxf(top[u], fabsf(p));
         add3(u, p, __fmaf_rn(a, b, -p), 0.0f);
@@ -367,12 +372,11 @@ __global__ void __launch_bounds__(256)
     };
     const int sj[3] = {d.nstart[1], d.nstart[2], d.nmax};
     for (int s = 0; s <= d.nmax; ++s) {
-        Dots<T, P> dot;
+        Dots<T, P, 4> dot;
         if (in) {
             const T* a = qf + s * sl + r;
             const T* c = qb + s * sl + r;
-#pragma unroll 4
-            for (int i = g; i < d.M; i += G) {
+            auto row = [&](int i, int k) {
                 T x[P], y[P];
                 if constexpr (P > 1) {
                     vload<T>(a + i * nr, x);
@@ -382,8 +386,14 @@ __global__ void __launch_bounds__(256)
                     y[0] = c[i * nr];
                 }
 #pragma unroll
-                for (int u = 0; u < P; ++u) dot.add(u, x[u], y[u]);
+                for (int u = 0; u < P; ++u) dot.add(u, x[u], y[u], k);
+            };
+            int i = g;
+            for (; i + 3 * G < d.M; i += 4 * G) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) row(i + k * G, k);
             }
+            for (; i < d.M; i += G) row(i, 0);
         }
         double v[P];
 #pragma unroll
