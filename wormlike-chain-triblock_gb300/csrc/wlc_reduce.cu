@@ -288,10 +288,11 @@ __global__ void __launch_bounds__(Pts<T>::THREADS)
 // a product and its error are exact in two floats and are added to a sum of
 // three floats by error-free additions (72 bits; the FP64 pipe has 1/64 of
 // the FP32 rate, and one multiply-add with its two conversions costs 192
-// clocks of a scheduler there against 24 here).  That holds while the largest
+// clocks of a scheduler there against 26 here).  That holds while the largest
 // product lies within 2^-90 .. 2^100: errors of smaller products, below 2^-149,
-// are then under 2^-59 of it and no sum overflows.  Otherwise (and for zeros
-// and not-a-numbers) holds() is false and dot_fp64 sums again in FP64.
+// are then under 2^-59 of it and no sum overflows; or while one factor is zero
+// throughout (most coefficients at the chain's ends).  Otherwise holds() is
+// false and dot_fp64 sums again in FP64.
 __device__ __forceinline__ float two_sum(float a, float b, float& err) {
     const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
     err = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
@@ -322,6 +323,7 @@ template <int P, int K> struct Dots<double, P, K> {
 template <int P, int K> struct Dots<float, P, K> {
     static constexpr int W = 3;
     float s[P] = {}, c[P] = {}, d[P] = {}, top[P] = {};  // top: largest product
+    unsigned abits = 0, bbits = 0;                       // bits set in any factor, at any point
     __device__ __forceinline__ void add3(int u, float p, float e, float f) {
         float t1, t2, t3;
         s[u] = two_sum(s[u], p, t1);
@@ -332,9 +334,14 @@ template <int P, int K> struct Dots<float, P, K> {
     __device__ __forceinline__ void add(int u, float a, float b, int = 0) {
         const float p = __fmul_rn(a, b);
         top[u] = fmaxf(top[u], fabsf(p));
+        abits |= __float_as_uint(a);
+        bbits |= __float_as_uint(b);
         add3(u, p, __fmaf_rn(a, b, -p), 0.0f);
     }
-    __device__ __forceinline__ bool holds(int u) const { return top[u] >= 0x1p-90f && top[u] <= 0x1p100f && s[u] == s[u]; }
+    __device__ __forceinline__ bool holds(int u) const {
+        const bool zero = abits << 1 == 0 || bbits << 1 == 0;
+        return s[u] == s[u] && (zero || (top[u] >= 0x1p-90f && top[u] <= 0x1p100f));
+    }
     __device__ __forceinline__ double get(int u) const { return (double)s[u] + ((double)c[u] + (double)d[u]); }
 };
 
