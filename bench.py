@@ -349,7 +349,8 @@ def run_ours(args, wl):
                 "bytes_per_launch": pb[dom], "avg_launch_ms": avg_ms, "kernel_share": share,
                 "binding_limit": ("pass B: issue and latency of 64-bit integer work (ncu); the HBM fraction is"
                                   " reported alongside") if bq == 8 else
-                                 "latency-bound shared-memory FFT stages (ncu: 8-18 % DRAM, ~10 % FMA pipe)",
+                                 "latency of pass B at 24 warps per SM, barriers and shared-memory queue of passes A"
+                                 " and C (ncu: 21-42 % DRAM, ~20 % FMA pipe)",
                 "step": {"algorithmic_bytes": b_step, "ms": step_ms,
                          "achieved_gbs": b_step / (step_ms / 1000.0) / 1e9,
                          "frac": b_step / (step_ms / 1000.0) / 1e9 / peak}}

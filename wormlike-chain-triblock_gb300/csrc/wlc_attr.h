@@ -39,10 +39,13 @@ template <typename K> inline cudaError_t smem_attr_once(K* fn, int bytes) {
 // Launch of a kernel that begins with dep_wait() below: with `chain` it may be
 // put in place while the kernel before it on the stream finishes (programmatic
 // dependent launch), which takes the launch latency between the passes of a
-// contour step off their chain.  chained_step: where that was faster -- short
-// kernels (iterations at 16^3, L = 2 FP64 4.87 -> 4.33 ms, 40^3, L = 7 FP32 10.6 ->
-// 9.85 ms); CTAs put in place early hold shared memory that the other sweep's
-// kernels could use (32^3, L = 6 FP64 27.2 -> 28.7 ms, 64^3 FP32 98.5 -> 99.4 ms).
+// contour step off their chain.  chained_step: where that was faster at every
+// degree.  Both sweeps and the density, chained against not, 17 pairs of grid
+// and degree in FP32 and 15 in FP64: FP32 16^3 .. 40^3 (L = 1 .. 12) 0.75-0.99
+// of the time, 48^3 0.88-1.01; FP64 8^3 .. 24^3 (L = 1 .. 10) 0.85-1.00.  Above,
+// CTAs put in place early hold shared memory that the other sweep's kernels
+// could use: FP64 32^3, L = 6 1.03, FP32 64^3, L = 10 1.01 (lower degrees there
+// would gain 2-9 %).
 #ifdef __CUDACC__
 __host__ __device__
 #endif

@@ -349,8 +349,9 @@ template <int P, int K> struct Dots<float, P, K> {
 // s = NA, NA+NB, Nmax; qend[r] = q_0(r, Nmax).  Every slice is read once.  A
 // CTA's threads are G groups of coefficients for 256 / G times P points; the
 // larger G serves grids that would not fill the SMs otherwise.
-// FP32, 64^3, L = 10, 101 slices (25.6 GB): 8.1 ms; with conversions and
-// multiply-adds on the FP64 pipe the iteration took 10.7 ms longer.
+// 64^3, L = 10, 101 slices, four rows of loads in flight: FP32 (25.6 GB) 5.6 ms
+// (8.0 row by row; with conversions and multiply-adds on the FP64 pipe 10.7
+// more), FP64 7.1 ms (7.2).
 template <typename T, int P, int G>
 __global__ void __launch_bounds__(256)
     density_accum(const T* __restrict__ qf, const T* __restrict__ qb, DensityArgs d, double* __restrict__ raw,
@@ -592,7 +593,8 @@ __global__ void __launch_bounds__(Pts<T>::THREADS)
 // issued by the backward sweep right after q*(s) is computed (descending s),
 // so the q* slices need not be stored.  Same Simpson weights per block.  One
 // CTA walks tiles of TILE points of one instance.
-// 128^3, L = 12 with the tensor in FP32: 9.9 -> 2.4 ms a launch.
+// 128^3, L = 12 with the tensor in FP32: 9.9 -> 2.5 ms a launch (2.4 without the
+// guard of the sums' range).
 template <typename T>
 __device__ __forceinline__ void density_slice_tiles(const T* __restrict__ a, const T* __restrict__ c,
                                                     const DensityArgs& d, int s, int want_s, const ClassLists& jl,

@@ -300,7 +300,9 @@ template <int N, int V = 0> __global__ void __launch_bounds__(512) ifft_xy(StepA
 // stay together).  Other J: natural order in rows of odd length, lanes
 // line-fastest.  Pass C: slot (j, k) at j S + k, S odd, so that neighbouring
 // lanes write >= 4 neighbours of a row.  Either way neighbouring lanes are on
-// distinct banks in both sub-passes.
+// distinct banks in both sub-passes.  (Pass A with the second radix first, every
+// row padded: 32^3, L = 8 18.4 us a launch against 17.5, 48^3 54.5 against 53.5,
+// 96^3, L = 6 272 against 267, the others within 1 %.)
 template <int N, bool FWD> struct XLine {
     static constexpr int R = Plan<N, float>::N1, J = Plan<N, float>::N2;
     static constexpr bool JFAST = J % 4 == 0;
